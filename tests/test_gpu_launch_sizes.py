@@ -4,7 +4,11 @@ A warp's first rays are its own by its number, spread over the grid's warps
 when the launch has fewer rays than the grid has lanes; later rays come from a
 counter.  Sizes at and around the edges of that rule (one ray, a warp, the
 grid's warps, its lanes) must give the oracle's hits bit for bit and write
-nothing past the last ray."""
+nothing past the last ray.
+
+Waves of at most 65,536 paths without shadow rays run whole in one launch;
+their images and ray counts must equal the staged launches' (which profiled
+frames use) and the megakernel's, below, at and above that size."""
 import numpy as np
 import pytest
 
@@ -41,3 +45,26 @@ def test_every_launch_size_gives_the_oracle_hits(scene, n, any_hit):
     got = d_hits.cpu().numpy()
     assert (got[n:] == GUARD).all()
     assert_hits_equal(got[:n].copy().view(want[0].dtype).reshape(n), want[int(any_hit)][:n], f"{n} rays")
+
+
+# 65,535 / 65,536 / 65,538 paths; a wave split into short ones; many samples; no bounce
+@pytest.mark.parametrize("width,height,spp,bounces,rr,wave", [
+    (1, 1, 1, 4, 99, 0), (257, 255, 1, 2, 99, 0), (256, 256, 1, 4, 3, 0), (10923, 6, 1, 1, 99, 0),
+    (97, 61, 5, 6, 2, 1000), (60, 40, 7, 0, 99, 0)])
+def test_whole_waves_equal_staged_launches(width, height, spp, bounces, rr, wave):
+    desc = scenes.mixed_box_scene(width, height)
+    kw = dict(max_bounces=bounces, spp=spp, nee=0, rr_start_depth=rr, wave_paths=wave, frame_seed=5)
+    with Renderer(width, height) as r:
+        load_scene_into(r, desc)
+        images, stats = [], []
+        for extra in (dict(), dict(profile=True), dict(megakernel=True)):
+            r.render(accumulate=False, **kw, **extra)
+            r.render(accumulate=True, **kw, **extra)   # a second call on top
+            images.append(r.read_image())
+            stats.append(r.stats())
+    assert width * height == 1 or bounces == 0 or images[0][..., :3].max() > 0.0   # the light is behind the camera
+    for k in (1, 2):
+        assert np.array_equal(images[0].view(np.uint32), images[k].view(np.uint32))
+        assert stats[0]["rays_extend"] == stats[k]["rays_extend"] and stats[0]["rays_connect"] == 0
+    assert stats[0]["extend_rays_depth"] == stats[1]["extend_rays_depth"]
+    assert (stats[0]["launches"] < stats[1]["launches"]) == ((wave or width * height * spp) <= 65536)

@@ -1326,6 +1326,19 @@ std::vector<Wave> plan_waves(uint32_t spp, uint32_t npix, uint32_t wave) {
     return waves;
 }
 
+// Waves of at most this many paths without shadow rays run whole in one
+// k_finish launch instead of an extend and a shade launch per depth.  us per
+// frame, staged / whole, frames of three contexts in flight (alone), box scene
+// depth 4: 4,096 paths 181 / 107 (374 / 228), 32,761: 252 / 185 (477 / 347),
+// 65,536: 299 / 235 (550 / 416), 131,044: 365 / 380 (652 / 617), 262,144:
+// 509 / 711; five spheres of every material, depth 8: 65,536: 554 / 495,
+// 131,072: 689 / 810.  (k_finish keeps 77,824 paths in flight: 4 blocks of 128
+// on each of 152 SMs.)  With shadow rays a path's own chain is twice as long
+// and the staged launches overlap their two kinds: from the first queue of at
+// most 65,536 paths on, finishing a wave measured 3-5 % slower there (613x377
+// textured frame 2.33 -> 2.40 ms, 720p frame 1.19 -> 1.23 ms).
+constexpr uint32_t kWholePaths = 65536;
+
 struct Pass {
     WaveParams W;
     SceneRefs S;
@@ -1456,10 +1469,17 @@ int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, const Adj
             if (projected < limit) { tail = d; break; }
         }
     }
+    // A short wave without shadow rays runs whole in one launch.
+    const bool whole = W.npaths <= kWholePaths && !P.nee && !P.prof && !P.cnt && P.S.qbvh == 0u && !A.g_albedo &&
+                       !B.ps_Lc && W.view_mode == 0u && P.tail_paths == 0u;
+    if (whole) {
+        WF_CUDA(launch_finish(P.S, P.SH, B, W, 0, c->totals, c->stream));
+        c->launches++;
+    }
     // generate.hlsl's camera rays are made inside the depth-0 traversal launch
     // and shade takes the starting path state at depth 0, so no pass writes them
     bool pending = false;   // a connect on the side stream not yet joined
-    for (uint32_t d = 0; d <= W.max_bounces; ++d) {
+    for (uint32_t d = 0; d <= W.max_bounces && !whole; ++d) {
         if (d == tail) {
             // connect at depth d - 1 has added its contributions first (also
             // under the fused schedule: no extension launch of this depth
@@ -1469,7 +1489,7 @@ int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, const Adj
                 pending = false;
             }
             StageTimer t(c, P.prof, ST_TAIL);
-            WF_CUDA(launch_megakernel_tail(P.S, P.SH, B, W, d, B.counts + 2 * kMaxDepth + d, c->totals, c->stream));
+            WF_CUDA(launch_finish(P.S, P.SH, B, W, d, c->totals, c->stream));
             c->launches++;
             c->tail_depth = d;
             break;
