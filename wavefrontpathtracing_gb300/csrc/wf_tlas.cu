@@ -3,13 +3,13 @@
 //
 // The reference's A/B/C walk is inherently sequential: each step asks
 // find_best_match (:86-110) for the partner of one node among the remaining
-// ones.  One warp runs the walk; every find_best_match is a warp-parallel scan
-// of the remaining list (each lane scans a strided slice in increasing order,
-// keeping its first strict minimum, then a shuffle reduction takes the
-// smallest value and, on equal values, the smallest list position — exactly
-// the element the reference's sequential "area < smallest" loop keeps).  The
-// remaining list and its boxes live in shared memory when they fit.
+// ones.  One block runs the walk; every find_best_match is a scan of the
+// remaining boxes by all its threads (each keeps its first strict minimum, then
+// warp reductions take the smallest value and, on equal values, the smallest
+// list position — exactly the element the reference's sequential "area <
+// smallest" loop keeps).
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/wf.h"
 #include "wf_kernels.h"
@@ -29,35 +29,88 @@ struct List {
     float* bmx;
 };
 
-// find_best_match: partner of list position X among positions [0, count).
-__device__ uint32_t best_match(const List& L, uint32_t X, uint32_t count, uint32_t metric) {
-    const uint32_t lane = threadIdx.x;
-    const float ax0 = L.bmn[3 * X], ax1 = L.bmn[3 * X + 1], ax2 = L.bmn[3 * X + 2];
-    const float bx0 = L.bmx[3 * X], bx1 = L.bmx[3 * X + 1], bx2 = L.bmx[3 * X + 2];
-    float best = FLT_MAX;
-    uint32_t bi = 0xFFFFFFFFu;
-    for (uint32_t j = lane; j < count; j += 32u) {
-        if (j == X) continue;
-        float hx, hy, hz, lx, ly, lz;
+// A float's bits in an unsigned order equal to float order (-0 below +0).
+__device__ __forceinline__ uint32_t sortable_bits(float x) {
+    const uint32_t u = __float_as_uint(x);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+struct Box {
+    float mn[3], mx[3];
+};
+
+// find_best_match's pairing value of two boxes.
+__device__ __forceinline__ float pair_area(const Box& A, const Box& B, uint32_t metric) {
+    float h[3], l[3];
+    for (int a = 0; a < 3; ++a) {
         if (metric == 0) {
             // the reference's corners: "max" = max(A.min, B.min), "min" = max(A.max, B.max)
-            hx = gmax(ax0, L.bmn[3 * j]); hy = gmax(ax1, L.bmn[3 * j + 1]); hz = gmax(ax2, L.bmn[3 * j + 2]);
-            lx = gmax(bx0, L.bmx[3 * j]); ly = gmax(bx1, L.bmx[3 * j + 1]); lz = gmax(bx2, L.bmx[3 * j + 2]);
+            h[a] = gmax(A.mn[a], B.mn[a]);
+            l[a] = gmax(A.mx[a], B.mx[a]);
         } else {
             // the merged box
-            lx = gmin(ax0, L.bmn[3 * j]); ly = gmin(ax1, L.bmn[3 * j + 1]); lz = gmin(ax2, L.bmn[3 * j + 2]);
-            hx = gmax(bx0, L.bmx[3 * j]); hy = gmax(bx1, L.bmx[3 * j + 1]); hz = gmax(bx2, L.bmx[3 * j + 2]);
+            l[a] = gmin(A.mn[a], B.mn[a]);
+            h[a] = gmax(A.mx[a], B.mx[a]);
         }
-        float ex = hx - lx, ey = hy - ly, ez = hz - lz;
-        float area = ex * ey + ey * ez + ez * ex;
+    }
+    const float ex = h[0] - l[0], ey = h[1] - l[1], ez = h[2] - l[2];
+    return ex * ey + ey * ez + ez * ex;
+}
+
+__device__ __forceinline__ Box list_box(const List& L, uint32_t j) {
+    Box b;
+    for (int a = 0; a < 3; ++a) { b.mn[a] = L.bmn[3 * j + a]; b.mx[a] = L.bmx[3 * j + a]; }
+    return b;
+}
+
+constexpr uint32_t kNoPos = 0xFFFFFFFFu;
+
+// The whole block's smallest value and, on equal values, lowest position of
+// (best, bi) over the threads (bi = kNoPos: none); every thread returns the
+// position and leaves the value in best.  Values compare as sortable bits with
+// -0 made +0, so equal floats are equal keys.  One barrier: two calls in a row
+// use the two halves of s_part.
+__device__ __forceinline__ uint32_t block_first_min(float& best, uint32_t bi, uint2 (*s_part)[32], uint32_t& buf) {
+    const uint32_t T = blockDim.x, t = threadIdx.x, lane = t & 31u;
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t key = bi == kNoPos ? 0xFFFFFFFFu : sortable_bits(best + 0.0f);
+    uint32_t k = __reduce_min_sync(FULL, key), i = __reduce_min_sync(FULL, key == k ? bi : kNoPos);
+    if (lane == 0) s_part[buf][t >> 5] = make_uint2(k, i);
+    __syncthreads();
+    const uint2 v = lane < (T >> 5) ? s_part[buf][lane] : make_uint2(0xFFFFFFFFu, kNoPos);
+    buf ^= 1u;
+    k = __reduce_min_sync(FULL, v.x);
+    i = __reduce_min_sync(FULL, v.x == k ? v.y : kNoPos);
+    best = __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
+    return i;
+}
+
+// find_best_match for the whole block: the partner of box Q (list position X)
+// among positions [0, count).  Thread t holds the boxes of positions t, t + T,
+// .. in registers (own[E], T = blockDim.x); positions past E T come from the
+// list.  Every thread returns the same position: the smallest value, on equal
+// values the lowest position (the element that the sequential "area <
+// smallest" loop keeps; a NaN is never below, as there).
+template <int E>
+__device__ __forceinline__ uint32_t best_match(const List& L, const Box (&own)[E], const Box& Q, uint32_t X,
+                                               uint32_t count, uint32_t metric, uint2 (*s_part)[32], uint32_t& buf) {
+    const uint32_t T = blockDim.x, t = threadIdx.x;
+    float best = FLT_MAX;
+    uint32_t bi = kNoPos;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t j = t + (uint32_t)e * T;
+        const float area = pair_area(Q, own[e], metric);
+        if (j < count && j != X && area < best) { best = area; bi = j; }
+    }
+    for (uint32_t j = t + (uint32_t)E * T; j < count; j += T) {
+        if (j == X) continue;
+        const float area = pair_area(Q, list_box(L, j), metric);
         if (area < best) { best = area; bi = j; }
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        float ob = __shfl_down_sync(0xffffffffu, best, off);
-        uint32_t oi = __shfl_down_sync(0xffffffffu, bi, off);
-        if (ob < best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    return __shfl_sync(0xffffffffu, bi, 0);
+    const uint32_t i = block_first_min(best, bi, s_part, buf);
+    // no value below FLT_MAX (not for finite boxes): any other position
+    return i != kNoPos ? i : (X == 0u ? 1u : 0u);
 }
 
 __device__ __forceinline__ void store_node(float4* nodes, uint32_t k, const float* mn, uint32_t lr, const float* mx,
@@ -66,56 +119,83 @@ __device__ __forceinline__ void store_node(float4* nodes, uint32_t k, const floa
     nodes[2 * k + 1] = make_float4(mx[0], mx[1], mx[2], __uint_as_float(inst));
 }
 
-// The reference's A/B/C walk (tlas_builder.cpp:18-67) for one warp.  aabbs:
-// 6 floats per instance (min xyz, max xyz); nodes: 2n nodes; base: the
-// working list, 7 words per instance (node index, box min, box max), in
-// shared memory, a scratch buffer or the allocation-free build's static array.
+// The reference's A/B/C walk (tlas_builder.cpp:18-67) for one block of T
+// threads, a multiple of 32, past k_tlas_walk's sizes.  aabbs: 6 floats per instance (min xyz, max xyz);
+// nodes: 2n nodes; base: the working list, 7 words per instance (node index,
+// box min, box max), in shared memory, a scratch buffer or the allocation-free
+// build's static array.
+template <int E>
 __device__ __forceinline__ void tlas_walk(const float* __restrict__ aabbs, uint32_t n, float4* nodes, uint32_t* base,
                                           uint32_t metric) {
+    __shared__ uint2 s_part[2][32];
     List L;
     L.idx = base;
     L.bmn = reinterpret_cast<float*>(base + n);
     L.bmx = reinterpret_cast<float*>(base + 4 * n);
-    const uint32_t lane = threadIdx.x;
-    for (uint32_t i = lane; i < n; i += 32u) {
+    const uint32_t T = blockDim.x, t = threadIdx.x;
+    for (uint32_t i = t; i < n; i += T) {
         float mn[3] = {aabbs[6 * i], aabbs[6 * i + 1], aabbs[6 * i + 2]};
         float mx[3] = {aabbs[6 * i + 3], aabbs[6 * i + 4], aabbs[6 * i + 5]};
         store_node(nodes, 1 + i, mn, 0u, mx, i);
         L.idx[i] = 1 + i;
         for (int a = 0; a < 3; ++a) { L.bmn[3 * i + a] = mn[a]; L.bmx[3 * i + a] = mx[a]; }
     }
-    __syncwarp();
-    uint32_t remaining = n, at = n + 1;
-    uint32_t A = 0;
-    uint32_t B = best_match(L, A, remaining, metric);
+    Box own[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t i = min(t + (uint32_t)e * T, n - 1u);
+        for (int a = 0; a < 3; ++a) { own[e].mn[a] = aabbs[6 * i + a]; own[e].mx[a] = aabbs[6 * i + 3 + a]; }
+    }
+    __syncthreads();
+    uint32_t remaining = n, at = n + 1, buf = 0;
+    uint32_t A = 0, steps = 0;
+    Box QA = list_box(L, A);
+    uint32_t B = best_match<E>(L, own, QA, A, remaining, metric, s_part, buf);
     while (remaining > 1) {
-        const uint32_t C = best_match(L, B, remaining, metric);
-        if (A == C) {
-            if (lane == 0) {
-                const uint32_t ia = L.idx[A], ib = L.idx[B];
-                float mn[3], mx[3];
-                for (int a = 0; a < 3; ++a) {
-                    mn[a] = gmin(L.bmn[3 * A + a], L.bmn[3 * B + a]);
-                    mx[a] = gmax(L.bmx[3 * A + a], L.bmx[3 * B + a]);
-                }
-                store_node(nodes, at, mn, ia + (ib << 16), mx, 0u);
-                L.idx[A] = at;
-                for (int a = 0; a < 3; ++a) { L.bmn[3 * A + a] = mn[a]; L.bmx[3 * A + a] = mx[a]; }
-                const uint32_t last = remaining - 1;
-                L.idx[B] = L.idx[last];
-                for (int a = 0; a < 3; ++a) { L.bmn[3 * B + a] = L.bmn[3 * last + a]; L.bmx[3 * B + a] = L.bmx[3 * last + a]; }
+        const Box QB = list_box(L, B);
+        const uint32_t C = best_match<E>(L, own, QB, B, remaining, metric, s_part, buf);
+        if (A == C || ++steps > n) {   // (steps: boxes of NaN have no order, see k_tlas_walk)
+            steps = 0;
+            // every thread forms the merged box; the list is written once all have read it
+            const uint32_t last = remaining - 1;
+            const Box QL = list_box(L, last);
+            const uint32_t ia = L.idx[A], ib = L.idx[B], il = L.idx[last];
+            Box M;
+            for (int a = 0; a < 3; ++a) {
+                M.mn[a] = gmin(QA.mn[a], QB.mn[a]);
+                M.mx[a] = gmax(QA.mx[a], QB.mx[a]);
             }
-            __syncwarp();
+            __syncthreads();
+            if (t == 0) {
+                store_node(nodes, at, M.mn, ia + (ib << 16), M.mx, 0u);
+                L.idx[A] = at;
+                for (int a = 0; a < 3; ++a) { L.bmn[3 * A + a] = M.mn[a]; L.bmx[3 * A + a] = M.mx[a]; }
+                // position B takes the last one (in that order, as the reference: B may be the last)
+                L.idx[B] = A == last ? at : il;
+                const Box& V = A == last ? M : QL;
+                for (int a = 0; a < 3; ++a) { L.bmn[3 * B + a] = V.mn[a]; L.bmx[3 * B + a] = V.mx[a]; }
+            }
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const uint32_t j = t + (uint32_t)e * T;
+                if (j == A) own[e] = M;
+                if (j == B) own[e] = A == last ? M : QL;
+            }
             at++;
             remaining--;
-            B = best_match(L, A, remaining, metric);
+            // the barrier in the next call orders the writes before the list's next
+            // reads, but for positions past the registers, which the call itself reads
+            if (remaining > (uint32_t)E * T) __syncthreads();
+            QA = M;
+            B = best_match<E>(L, own, QA, A, remaining, metric, s_part, buf);
         } else {
             A = B;
+            QA = QB;
             B = C;
         }
     }
-    __syncwarp();
-    if (lane == 0) {
+    __syncthreads();
+    if (t == 0) {
         const uint32_t r = L.idx[A];
         const float4 a = nodes[2 * r], b = nodes[2 * r + 1];
         nodes[0] = a;
@@ -123,11 +203,198 @@ __device__ __forceinline__ void tlas_walk(const float* __restrict__ aabbs, uint3
     }
 }
 
-// One warp; the list in shared memory when it fits, else in gscratch.
-__global__ void __launch_bounds__(32) k_tlas_build(const float* __restrict__ aabbs, uint32_t n, float4* nodes,
-                                                   uint32_t* gscratch, uint32_t metric) {
+// The same walk for n <= E T: every remaining box is in a register slot
+// (position e T + t in thread t's slot e; an empty slot holds the box from
+// -inf to +inf, whose value against any box is +inf or NaN under either
+// metric, never below), so a find_best_match reads one box from the list and scans
+// registers.  Few warps and many slots: what a call costs besides the scan (the
+// box, the reduction, the barrier) is paid by every warp.
+//
+// Bound by the latency of a call, about 0.37 us at 1,025 instances (4,376 calls
+// in sequence; two warp reductions, a barrier, the box's load).  us per
+// wf_tlas_build, metric 0, one warp scanning a list in shared memory / here:
+// 64 instances 159 / 84, 256: 866 / 311, 1,025: 7,918 / 1,628, 4,096: 105,057 /
+// 13,385.  Keeping every position's partner up to date instead of scanning
+// (each merge one evaluation per box) measured 4,157 us at 1,025: a merge
+// invalidates 2.8 partners that the walk then asks for.
+template <int E, int T, uint32_t metric>
+__global__ void __launch_bounds__(T) k_tlas_walk(const float* __restrict__ aabbs, uint32_t n, float4* nodes,
+                                                 uint32_t* gscratch, uint32_t, int in_smem) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    constexpr uint32_t W = T / 32;
+    __shared__ unsigned long long s_part[2][W];
+    // per position: {box min, node index}, {box max, -}
+    float4* L = reinterpret_cast<float4*>(in_smem ? smem : gscratch);
+    const uint32_t t = threadIdx.x, lane = t & 31u;
+    const unsigned FULL = 0xffffffffu;
+    const float inf = __uint_as_float(0x7F800000u);
+    for (uint32_t i = t; i < n; i += T) {
+        float mn[3] = {aabbs[6 * i], aabbs[6 * i + 1], aabbs[6 * i + 2]};
+        float mx[3] = {aabbs[6 * i + 3], aabbs[6 * i + 4], aabbs[6 * i + 5]};
+        store_node(nodes, 1 + i, mn, 0u, mx, i);
+        L[2 * i] = make_float4(mn[0], mn[1], mn[2], __uint_as_float(1u + i));
+        L[2 * i + 1] = make_float4(mx[0], mx[1], mx[2], 0.0f);
+    }
+    auto entry = [&](uint32_t j, uint32_t& id) {
+        const float4 a = L[2 * j], b = L[2 * j + 1];
+        id = __float_as_uint(a.w);
+        return Box{{a.x, a.y, a.z}, {b.x, b.y, b.z}};
+    };
+    Box own[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t j = t + (uint32_t)(e * T);
+        for (int a = 0; a < 3; ++a) {
+            own[e].mn[a] = j < n ? aabbs[6 * j + a] : -inf;
+            own[e].mx[a] = j < n ? aabbs[6 * j + 3 + a] : inf;
+        }
+    }
+    // slot of position j (in its thread) takes box V
+    auto put = [&](uint32_t j, const Box& V) {
+        if (t != j % T) return;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const bool here = (uint32_t)e == j / T;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                own[e].mn[a] = here ? V.mn[a] : own[e].mn[a];
+                own[e].mx[a] = here ? V.mx[a] : own[e].mx[a];
+            }
+        }
+    };
+    uint32_t buf = 0;
+    auto best_match = [&](const Box& Q, uint32_t X, uint32_t count) -> uint32_t {
+        const uint32_t xe = t == X % T ? X / T : kNoPos;   // X's own slot is no candidate
+        float best = FLT_MAX;
+        uint32_t be = kNoPos;
+        auto scan = [&](auto slots) {
+#pragma unroll
+            for (int e = 0; e < decltype(slots)::value; ++e) {
+                const float area = pair_area(Q, own[e], metric);
+                if (area < best && (uint32_t)e != xe) { best = area; be = (uint32_t)e; }
+            }
+        };
+        // straight-line scans: with a warp or two per scheduler a branch per slot costs more than the slot
+        if (E >= 4 && count <= (uint32_t)(E / 4 * T)) scan(std::integral_constant<int, E / 4>{});
+        else if (E >= 2 && count <= (uint32_t)(E / 2 * T)) scan(std::integral_constant<int, E / 2>{});
+        else scan(std::integral_constant<int, E>{});
+        const uint32_t bi = be == kNoPos ? kNoPos : be * T + t;
+        const uint32_t key = be == kNoPos ? 0xFFFFFFFFu : sortable_bits(best + 0.0f);   // -0 as +0
+        const uint32_t k = __reduce_min_sync(FULL, key), i = __reduce_min_sync(FULL, key == k ? bi : kNoPos);
+        uint32_t r = i;
+        if (W > 1) {
+            if (lane == 0) s_part[buf][t >> 5] = ((unsigned long long)k << 32) | i;
+            __syncthreads();
+            unsigned long long m = s_part[buf][0];
+#pragma unroll
+            for (uint32_t w = 1; w < W; ++w) m = min(m, s_part[buf][w]);
+            buf ^= 1u;   // the next call's partials go to the other half: one barrier per call
+            r = (uint32_t)m;
+        } else {
+            __syncwarp();
+        }
+        // no value below FLT_MAX (not for finite boxes): any other position
+        return r != kNoPos ? r : (X == 0u ? 1u : 0u);
+    };
+    __syncthreads();
+    uint32_t remaining = n, at = n + 1, A = 0, steps = 0, ia = 0, ib = 0, il = 0;
+    Box QA = entry(A, ia);
+    uint32_t B = best_match(QA, A, remaining);
+    while (remaining > 1) {
+        const Box QB = entry(B, ib);
+        const uint32_t C = best_match(QB, B, remaining);
+        // values fall (or positions do) along the walk, so it meets a mutual pair
+        // within a list's length; boxes of NaN, which have no order, merge there
+        if (A != C && ++steps <= n) {
+            A = B;
+            QA = QB;
+            ia = ib;
+            B = C;
+            continue;
+        }
+        steps = 0;
+        // every thread forms the merged box; the list is written once all have read it
+        const uint32_t last = remaining - 1;
+        const Box QL = entry(last, il);
+        Box M;
+        for (int a = 0; a < 3; ++a) {
+            M.mn[a] = gmin(QA.mn[a], QB.mn[a]);
+            M.mx[a] = gmax(QA.mx[a], QB.mx[a]);
+        }
+        // A becomes the merged box, then B the last position's (which A may be)
+        const Box VB = A == last ? M : QL;
+        put(A, M);
+        put(B, VB);
+        put(last, Box{{-inf, -inf, -inf}, {inf, inf, inf}});
+        __syncthreads();
+        if (t == 0) {
+            store_node(nodes, at, M.mn, ia + (ib << 16), M.mx, 0u);
+            L[2 * A] = make_float4(M.mn[0], M.mn[1], M.mn[2], __uint_as_float(at));
+            L[2 * A + 1] = make_float4(M.mx[0], M.mx[1], M.mx[2], 0.0f);
+            L[2 * B] = make_float4(VB.mn[0], VB.mn[1], VB.mn[2], __uint_as_float(A == last ? at : il));
+            L[2 * B + 1] = make_float4(VB.mx[0], VB.mx[1], VB.mx[2], 0.0f);
+        }
+        // (the barrier in the next call orders these writes before the list's next reads)
+        ia = at;
+        at++;
+        remaining--;
+        QA = M;
+        B = best_match(QA, A, remaining);
+    }
+    if (t == 0) {
+        const float4 a = nodes[2 * ia], b = nodes[2 * ia + 1];
+        nodes[0] = a;
+        nodes[1] = b;
+    }
+}
+
+constexpr uint32_t kScanThreads = 1024;
+
+// Past k_tlas_walk's sizes: the list in shared memory when it fits, else in gscratch.
+template <int E>
+__global__ void __launch_bounds__(kScanThreads) k_tlas_build(const float* __restrict__ aabbs, uint32_t n,
+                                                             float4* nodes, uint32_t* gscratch, uint32_t metric,
+                                                             int in_smem) {
     extern __shared__ uint32_t smem[];
-    tlas_walk(aabbs, n, nodes, (n <= kSmemInstances) ? smem : gscratch, metric);
+    tlas_walk<E>(aabbs, n, nodes, in_smem ? smem : gscratch, metric);
+}
+
+// The walk's launch.  scratch: 7 n words (8 n up to 4,096 instances), used when
+// the list does not fit shared memory (or when smem_ok is false).
+template <class K>
+cudaError_t launch_walk_kernel(K kernel, unsigned T, uint32_t words, const float* aabbs, uint32_t n, float4* nodes,
+                               uint32_t* scratch, uint32_t metric, bool smem_ok, cudaStream_t stream) {
+    const bool in_smem = smem_ok && n <= kSmemInstances;
+    const size_t smem = in_smem ? (size_t)n * words * 4u : 0u;
+    if (smem > 48u * 1024u) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    kernel<<<1, T, smem, stream>>>(aabbs, n, nodes, scratch, metric, in_smem ? 1 : 0);
+    return cudaGetLastError();
+}
+template <uint32_t metric>
+cudaError_t launch_walk(const float* aabbs, uint32_t n, float4* nodes, uint32_t* scratch, bool smem_ok,
+                        cudaStream_t st) {
+    auto walk = [&](auto kernel, unsigned threads) {
+        return launch_walk_kernel(kernel, threads, 8u, aabbs, n, nodes, scratch, metric, smem_ok, st);
+    };
+    // threads by size: us at 64 / 1,025 / 2,048 instances with 32 threads 84 / - / -,
+    // 128: 94 / 1,632 / 4,651, 192: 95 / 1,755 / 4,873, 256: 110 / 1,758 / 4,440
+    switch (n <= 64 ? (n + 31) / 32 : n <= 1536 ? 100 + (n + 127) / 128 : 0) {
+        case 1: return walk(k_tlas_walk<1, 32, metric>, 32);
+        case 2: return walk(k_tlas_walk<2, 32, metric>, 32);
+        case 101: return walk(k_tlas_walk<1, 128, metric>, 128);
+        case 102: return walk(k_tlas_walk<2, 128, metric>, 128);
+        case 103: case 104: return walk(k_tlas_walk<4, 128, metric>, 128);
+        case 105: case 106: return walk(k_tlas_walk<6, 128, metric>, 128);
+        case 107: case 108: return walk(k_tlas_walk<8, 128, metric>, 128);
+        case 109: case 110: return walk(k_tlas_walk<10, 128, metric>, 128);
+        case 111: case 112: return walk(k_tlas_walk<12, 128, metric>, 128);
+    }
+    if (n <= 2048) return walk(k_tlas_walk<8, 256, metric>, 256);
+    if (n <= 4096) return walk(k_tlas_walk<16, 256, metric>, 256);
+    return launch_walk_kernel(k_tlas_build<4>, kScanThreads, 7u, aabbs, n, nodes, scratch, metric, smem_ok, st);
 }
 
 }  // namespace
@@ -394,11 +661,6 @@ __global__ void __launch_bounds__(kPlocThreads) k_tlas_ploc(const float* __restr
 // n + 1 + k (every boundary is split once), so node numbers do not depend on
 // which warp takes which range; a child sets its half of the parent's
 // left_right word.  Identical, node for node, to the oracle's tlas_sweep.
-__device__ __forceinline__ uint32_t sortable_bits(float x) {
-    const uint32_t u = __float_as_uint(x);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
 constexpr uint32_t kSweepSmemMax = 2048;
 
 // Boxes live as sortable bits (an unsigned order equal to float order, -0
@@ -1178,13 +1440,8 @@ cudaError_t launch_tlas_build(const float* aabbs, uint32_t n, float4* nodes, uin
         k_tlas_sweep<<<1, kPlocThreads, bytes, stream>>>(aabbs, n, nodes, scratch, P, smem);
         return cudaGetLastError();
     }
-    size_t smem = (n <= kSmemInstances) ? (size_t)n * 7u * 4u : 0u;
-    if (smem > 48u * 1024u) {
-        cudaError_t e = cudaFuncSetAttribute(k_tlas_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    k_tlas_build<<<1, 32, smem, stream>>>(aabbs, n, nodes, scratch, metric);
-    return cudaGetLastError();
+    return metric == 0 ? launch_walk<0>(aabbs, n, nodes, scratch, true, stream)
+                       : launch_walk<1>(aabbs, n, nodes, scratch, true, stream);
 }
 
 // ============================================================================
@@ -1231,13 +1488,6 @@ CtxGetCurrentFn ctx_get_current() {
         return reinterpret_cast<CtxGetCurrentFn>(f);
     }();
     return fn;
-}
-
-// The walk of k_tlas_build with the list in the static array (`list` is its
-// device address).
-__global__ void __launch_bounds__(32) k_tlas_build_noalloc(const float* __restrict__ aabbs, uint32_t n,
-                                                           float4* nodes, uint32_t* list, uint32_t metric) {
-    tlas_walk(aabbs, n, nodes, list, metric);
 }
 
 }  // namespace
@@ -1290,9 +1540,10 @@ extern "C" int wf_tlas_build_noalloc(const float* device_aabbs, uint32_t instanc
     if (instance_count == 0) {
         e = cudaMemsetAsync(device_nodes, 0, 32, st);   // one zero node, as tlas_builder_t leaves it
     } else {
-        k_tlas_build_noalloc<<<1, 32, 0, st>>>(device_aabbs, instance_count, static_cast<float4*>(device_nodes),
-                                                list, tlas_metric);
-        e = cudaGetLastError();
+        // the walk with the list in the static array, by its device address
+        float4* nodes = static_cast<float4*>(device_nodes);
+        e = tlas_metric == 0 ? launch_walk<0>(device_aabbs, instance_count, nodes, list, false, st)
+                             : launch_walk<1>(device_aabbs, instance_count, nodes, list, false, st);
     }
     if (e != cudaSuccess) return report_error(WF_ERR_CUDA, cudaGetErrorString(e));
     return WF_OK;
