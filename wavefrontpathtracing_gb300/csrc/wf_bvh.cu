@@ -111,84 +111,8 @@ __device__ __forceinline__ bool goes_left(const Ctx& C, const Plan& P, uint32_t 
     return goes_left_c(C, P, comp(C.cen[t], P.axis));
 }
 
-// find_best_split_plane's sweep (bvh_builder.cpp:196-249) over bins laid out
-// [axis][bin][count, min xyz key, max xyz key].
-__device__ float sah_sweep(const uint32_t* bins, uint32_t B, const float* cmn, const float* cmx, uint32_t& axis,
-                           uint32_t& pos) {
-    float cheapest = FLT_MAX;
-    float larea[kMaxBins], rarea[kMaxBins];
-    for (uint32_t a = 0; a < 3; ++a) {
-        if (cmn[a] == cmx[a]) continue;
-        const uint32_t* ab = bins + a * B * kBinWords;
-        float lmn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, lmx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        float rmn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, rmx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        uint32_t lsum = 0, rsum = 0;
-        for (uint32_t i = 0; i < B - 1; ++i) {
-            const uint32_t* lb = ab + i * kBinWords;
-            lsum += lb[0];
-            for (int k = 0; k < 3; ++k) {
-                lmn[k] = gmin(lmn[k], fdec(lb[1 + k]));
-                lmx[k] = gmax(lmx[k], fdec(lb[4 + k]));
-            }
-            larea[i] = (float)lsum * half_area(lmn, lmx);
-            const uint32_t* rb = ab + (B - 1 - i) * kBinWords;
-            rsum += rb[0];
-            for (int k = 0; k < 3; ++k) {
-                rmn[k] = gmin(rmn[k], fdec(rb[1 + k]));
-                rmx[k] = gmax(rmx[k], fdec(rb[4 + k]));
-            }
-            rarea[B - 2 - i] = (float)rsum * half_area(rmn, rmx);
-        }
-        for (uint32_t i = 0; i < B - 1; ++i) {
-            float cost = larea[i] + rarea[i];
-            if (cost < cheapest) { axis = a; pos = i + 1; cheapest = cost; }
-        }
-    }
-    return cheapest;
-}
-
-// subdivide_node's decision (bvh_builder.cpp:104-118, 139-143) plus the
-// max_leaf_prims extension, without the split position p (which needs the
-// element at position nL: the caller places it).
-__device__ Plan make_plan_bins(const Ctx& C, const uint32_t* bins, uint32_t count, const float* nmn,
-                               const float* nmx, const float* cmn, const float* cmx) {
-    Plan P{};
-    uint32_t axis = 0, pos = 0;
-    float cost = sah_sweep(bins, C.bins, cmn, cmx, axis, pos);
-    bool leaf;
-    if (C.single) {
-        leaf = count == 1;
-    } else {
-        bool force = C.max_leaf > 0 && count > C.max_leaf;
-        float parent = (float)count * half_area(nmn, nmx);
-        leaf = !force && cost >= parent;
-    }
-    P.axis = axis;
-    P.pos = pos;
-    P.partition = leaf ? 0u : 1u;
-    if (leaf) return P;
-    P.lo = cmn[axis];
-    P.scale = pos > 0 ? (float)C.bins / (cmx[axis] - cmn[axis]) : 0.0f;
-    uint32_t nl = 0;
-    if (pos > 0) {
-        const uint32_t* ab = bins + axis * C.bins * kBinWords;
-        for (uint32_t b = 0; b < pos; ++b) nl += ab[b * kBinWords];
-    }
-    P.nl = nl;
-    P.p = count;
-    P.children = (nl > 0 && nl < count) ? 1u : 0u;
-    return P;
-}
-
-// The same, reading the element at nL from the position list.
-__device__ Plan make_plan(const Ctx& C, const uint32_t* bins, uint32_t first, uint32_t count, const float* nmn,
-                          const float* nmx, const float* cmn, const float* cmx) {
-    Plan P = make_plan_bins(C, bins, count, nmn, nmx, cmn, cmx);
-    if (P.partition && P.nl < count) P.p = P.nl + (goes_left(C, P, C.idx[first + P.nl]) ? 0u : 1u);
-    return P;
-}
-
-// Warp-parallel form of sah_sweep for the small phase: every lane returns the
+// find_best_split_plane's sweep (bvh_builder.cpp:196-249) by one warp over bins
+// laid out [axis][bin][count, min xyz key, max xyz key]: every lane returns the
 // same (cheapest, axis, pos) and nl = the triangles in bins [0, pos).  Lane l
 // holds bins [q*l, q*l + q) (q = 1 for up to 32 bins, else 2); shuffle scans
 // give each plane its left prefix and right suffix.  Prefix and suffix boxes
@@ -294,13 +218,12 @@ __device__ float warp_sweep(const uint32_t* bins, uint32_t B, const float* cmn, 
     return cheapest;
 }
 
-// make_plan_bins for a whole warp over shared-memory bins (all lanes return
-// the same plan, p not yet placed).
-__device__ Plan make_plan_warp(const Ctx& C, const uint32_t* bins, uint32_t count, const float* nmn,
-                               const float* nmx, const float* cmn, const float* cmx, uint32_t lane) {
+// The plan of a node from its cheapest plane (p placed only where every
+// triangle goes one way).
+__device__ __forceinline__ Plan plan_from(const Ctx& C, float cost, uint32_t axis, uint32_t pos, uint32_t nl,
+                                          uint32_t count, const float* nmn, const float* nmx, const float* cmn,
+                                          const float* cmx) {
     Plan P{};
-    uint32_t axis, pos, nl;
-    const float cost = warp_sweep(bins, C.bins, cmn, cmx, lane, axis, pos, nl);
     bool leaf;
     if (C.single) {
         leaf = count == 1;
@@ -313,8 +236,9 @@ __device__ Plan make_plan_warp(const Ctx& C, const uint32_t* bins, uint32_t coun
     P.pos = pos;
     P.partition = leaf ? 0u : 1u;
     if (leaf) return P;
-    P.lo = cmn[axis];
-    P.scale = pos > 0 ? (float)C.bins / (cmx[axis] - cmn[axis]) : 0.0f;
+    const float lo = axis == 0 ? cmn[0] : axis == 1 ? cmn[1] : cmn[2], hi = axis == 0 ? cmx[0] : axis == 1 ? cmx[1] : cmx[2];
+    P.lo = lo;
+    P.scale = pos > 0 ? (float)C.bins / (hi - lo) : 0.0f;
     P.nl = pos > 0 ? nl : 0u;
     P.p = count;
     P.children = (P.nl > 0 && P.nl < count) ? 1u : 0u;
@@ -558,8 +482,9 @@ __global__ void __launch_bounds__(kChunkThreads) k_bin_chunks(Ctx C, Level Lv) {
     }
 }
 
+// A warp per slot.
 __global__ void k_plan(Ctx C, Level Lv) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (s >= Lv.nslots) return;
     const uint32_t t = Lv.slot_tmp[s];
     const uint32_t* key = Lv.slot_box + kBoxWords * s;
@@ -572,9 +497,16 @@ __global__ void k_plan(Ctx C, Level Lv) {
     const float* nmn = box;
     const float* nmx = box + 3;
     const uint32_t first = __float_as_uint(C.ta[t].w), count = __float_as_uint(C.tb[t].w);
-    C.ta[t] = make_float4(nmn[0], nmn[1], nmn[2], __uint_as_float(first));
-    C.tb[t] = make_float4(nmx[0], nmx[1], nmx[2], __uint_as_float(count));
-    Lv.plan[s] = make_plan(C, Lv.bins + (size_t)s * 3 * C.bins * kBinWords, first, count, nmn, nmx, cmn, cmx);
+    uint32_t axis, pos, nl;
+    const float cost = warp_sweep(Lv.bins + (size_t)s * 3 * C.bins * kBinWords, C.bins, cmn, cmx, lane, axis, pos, nl);
+    Plan P = plan_from(C, cost, axis, pos, nl, count, nmn, nmx, cmn, cmx);
+    // the element at position nl decides where the front part ends
+    if (P.partition && P.nl < count) P.p = P.nl + (goes_left(C, P, C.idx[first + P.nl]) ? 0u : 1u);
+    if (lane == 0) {
+        C.ta[t] = make_float4(nmn[0], nmn[1], nmn[2], __uint_as_float(first));
+        C.tb[t] = make_float4(nmx[0], nmx[1], nmx[2], __uint_as_float(count));
+        Lv.plan[s] = P;
+    }
 }
 
 // Block-wide exclusive prefix of a flag (blockDim.x <= 1024); returns the prefix
@@ -727,184 +659,298 @@ __global__ void __launch_bounds__(kChunkThreads) k_child_bounds(Ctx C, Level Lv)
 }
 
 // ---------------------------------------------------------------- small-subtree phase
-// One warp (one CTA) builds a whole subtree of at most kSmall triangles with
-// the subtree held in shared memory: each triangle's centroid, min and max
-// corner (component k of local triangle j at d[k * kSmall + j]), its index,
-// and a 16-bit permutation of local triangles that the partitions reorder.
-// Only the node records and the final index list go to global memory.  Node
-// ids come from one reservation of 2 * (count - 1) per subtree (a subtree of
-// count triangles splits at most count - 1 times); ids a subtree does not use
-// keep tdepth = kNone and are skipped by the renumbering.  The warp descends
-// into the smaller child and keeps the larger on a lane-distributed stack, so
-// at most log2(kSmall) + 1 entries are pending.
+// One CTA of kSmallWarps warps builds a whole subtree of at most kSmall
+// triangles with the subtree held in shared memory: each triangle's centroid,
+// min and max corner (component k of local triangle j at d[k * kSmall + j]),
+// its index, and a 16-bit permutation of local triangles that the partitions
+// reorder.  The subtree grows level by level: a warp per node, the children
+// listed for the next level, one barrier between levels.  Only the node records
+// and the final index list go to global memory.  Node ids come from one
+// reservation of 2 * (count - 1) per subtree (a subtree of count triangles
+// splits at most count - 1 times); ids a subtree does not use keep tdepth =
+// kNone and are skipped by the renumbering.
+//
+// What bounds it: instructions per node (and, in small meshes with few
+// subtrees, the latency of a node times the subtree's depth).  Most nodes hold
+// few triangles, so nodes of at most kDirect triangles skip the bins: a lane
+// per (axis, triangle) sums the two sides of the plane after its triangle's bin
+// over the node's triangles.  Only those planes can be the first minimum: the
+// planes behind them with no triangle in between have the same sides and a
+// higher number, and a plane with an empty side costs NaN.
+#ifndef WF_BVH_SMALL_WARPS
+#define WF_BVH_SMALL_WARPS 4
+#endif
+constexpr uint32_t kSmallWarps = WF_BVH_SMALL_WARPS;
+constexpr uint32_t kDirect = 10;   // 3 axes x 10 triangles: one lane each
+
 struct SmallSmem {
     float* d;
     uint32_t* oidx;
     uint16_t *perm, *ptmp, *F, *G;
-    uint32_t* bins;
+    uint32_t* task[2];   // nodes of a level: first | count << 8 | (id's offset in the reservation + 1) << 16
+    uint32_t* bins;      // per warp
 };
+static_assert(kSmall <= 128, "task words hold 8-bit counts and first positions");
 
 __host__ __device__ constexpr size_t small_smem_bytes(uint32_t bins) {
-    return (9ull + 1ull) * 4ull * kSmall + 4ull * 2ull * kSmall + 4ull * 3ull * bins * kBinWords;
+    return (9ull + 1ull + 2ull) * 4ull * kSmall + 4ull * 2ull * kSmall + 4ull * 3ull * bins * kBinWords * kSmallWarps;
 }
 
-__global__ void __launch_bounds__(32) k_small(Ctx C, uint32_t nsmall, uint32_t tcap) {
+// Warp-wide bounds from per-lane folds: v = node min / max, centroid min / max.
+__device__ __forceinline__ void box_warp_redux(float* v) {
+#pragma unroll
+    for (int k = 0; k < 12; ++k)
+        v[k] = fdec((k % 6) < 3 ? __reduce_min_sync(0xffffffffu, fenc(v[k])) : __reduce_max_sync(0xffffffffu, fenc(v[k])));
+}
+
+// The cheapest plane of a node of c <= kDirect triangles (see above): what
+// warp_sweep returns over the node's bins.
+__device__ __forceinline__ float direct_sweep(const SmallSmem& S, uint32_t B, uint32_t f, uint32_t c, const float* cmn,
+                                              const float* cmx, uint32_t lane, uint32_t& axis, uint32_t& pos,
+                                              uint32_t& nl) {
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t a = lane / kDirect, i = lane - a * kDirect;
+    const float lo = a == 0 ? cmn[0] : a == 1 ? cmn[1] : cmn[2], hi = a == 0 ? cmx[0] : a == 1 ? cmx[1] : cmx[2];
+    const bool valid = a < 3 && i < c && lo != hi;
+    uint32_t bin = 0;
+    if (valid) {
+        int32_t b = (int32_t)((S.d[a * kSmall + S.perm[f + i]] - lo) * ((float)B / (hi - lo)));
+        if ((int32_t)B - 1 < b) b = (int32_t)B - 1;
+        bin = (uint32_t)b;
+    }
+    float l[6], r[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) l[k] = r[k] = k < 3 ? FLT_MAX : -FLT_MAX;
+    uint32_t lc = 0;
+    for (uint32_t k = 0; k < c; ++k) {
+        const uint32_t j = S.perm[f + k];
+        const uint32_t kb = __shfl_sync(FULL, bin, a < 3 ? a * kDirect + k : 0u);
+        const bool left = kb <= bin;
+        lc += left ? 1u : 0u;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const float e = S.d[(3 + q) * kSmall + j];
+            const float none = q < 3 ? FLT_MAX : -FLT_MAX;
+            l[q] = q < 3 ? fminf(l[q], left ? e : none) : fmaxf(l[q], left ? e : none);
+            r[q] = q < 3 ? fminf(r[q], left ? none : e) : fmaxf(r[q], left ? none : e);
+        }
+    }
+    const float cost = (float)lc * half_area(l, l + 3) + (float)(c - lc) * half_area(r, r + 3);
+    const uint32_t key = valid && lc < c && cost < FLT_MAX ? fenc(cost + 0.0f) : kNone;
+    const uint32_t best = __reduce_min_sync(FULL, key);
+    axis = pos = nl = 0;
+    if (best == kNone) return FLT_MAX;
+    const uint32_t code = (a << 8) | bin;
+    const uint32_t first = __reduce_min_sync(FULL, key == best ? code : kNone);
+    const int src = __ffs(__ballot_sync(FULL, key == best && code == first)) - 1;
+    axis = first >> 8;
+    pos = (first & 0xFFu) + 1u;
+    nl = __shfl_sync(FULL, lc, src);
+    return fdec(best);
+}
+
+// One warp, one node (positions [f, f + c) of the subtree): its record, its
+// split, and the partition of its positions.  Returns nl, the left child's
+// triangles (0: no children).
+__device__ __forceinline__ uint32_t small_node(const Ctx& C, const SmallSmem& S, uint32_t* bins, uint32_t X,
+                                               uint32_t gfirst, uint32_t f, uint32_t c, uint32_t dep, uint32_t lane) {
+    // node bounds, centroid bounds and first zero positions
+    float v[12];
+    uint32_t zp[6];
+    box_init(v);
+    zero_init(zp);
+    for (uint32_t i = lane; i < c; i += 32) {
+        const uint32_t j = S.perm[f + i];
+        float e[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) e[k] = S.d[k * kSmall + j];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            v[a] = fminf(v[a], e[3 + a]);
+            v[3 + a] = fmaxf(v[3 + a], e[6 + a]);
+            v[6 + a] = fminf(v[6 + a], e[a]);
+            v[9 + a] = fmaxf(v[9 + a], e[a]);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            if (e[3 + k] == 0.0f && zp[k] == kNone) zp[k] = i;
+    }
+    box_warp_redux(v);
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        if (v[k] == 0.0f) {
+            const uint32_t z = __reduce_min_sync(0xffffffffu, zp[k]);
+            if (z != kNone) v[k] = S.d[(3 + k) * kSmall + S.perm[f + z]];
+        }
+    if (lane == 0) {
+        C.ta[X] = make_float4(v[0], v[1], v[2], __uint_as_float(gfirst + f));
+        C.tb[X] = make_float4(v[3], v[4], v[5], __uint_as_float(c));
+        C.tleft[X] = kNone;
+        C.tdepth[X] = dep;
+    }
+    uint32_t axis, pos, nl;
+    float cost;
+    if (c <= kDirect) {
+        cost = direct_sweep(S, C.bins, f, c, v + 6, v + 9, lane, axis, pos, nl);
+    } else {
+        bool deg[3];
+        float lo[3], scale[3];
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = v[6 + a];
+            deg[a] = v[6 + a] == v[9 + a];
+            scale[a] = deg[a] ? 0.0f : (float)C.bins / (v[9 + a] - v[6 + a]);
+        }
+        bins_reset(bins, 3 * C.bins * kBinWords, lane, 32);
+        __syncwarp();
+        for (uint32_t i = lane; i < c; i += 32) {
+            const uint32_t j = S.perm[f + i];
+            for (uint32_t a = 0; a < 3; ++a) {
+                if (deg[a]) continue;
+                int32_t bin = (int32_t)((S.d[a * kSmall + j] - lo[a]) * scale[a]);
+                if ((int32_t)C.bins - 1 < bin) bin = (int32_t)C.bins - 1;
+                uint32_t* e = bins + (a * C.bins + (uint32_t)bin) * kBinWords;
+                atomicAdd(&e[0], 1u);
+                atomicMin(&e[1], fenc(S.d[3 * kSmall + j]));
+                atomicMin(&e[2], fenc(S.d[4 * kSmall + j]));
+                atomicMin(&e[3], fenc(S.d[5 * kSmall + j]));
+                atomicMax(&e[4], fenc(S.d[6 * kSmall + j]));
+                atomicMax(&e[5], fenc(S.d[7 * kSmall + j]));
+                atomicMax(&e[6], fenc(S.d[8 * kSmall + j]));
+            }
+        }
+        __syncwarp();
+        cost = warp_sweep(bins, C.bins, v + 6, v + 9, lane, axis, pos, nl);
+    }
+    Plan P = plan_from(C, cost, axis, pos, nl, c, v, v + 3, v + 6, v + 9);
+    if (!P.partition) return 0;
+    // the closed form of the two-pointer partition (see the file head),
+    // positions relative to the node's first position f
+    if (P.nl < c) P.p = P.nl + (goes_left_c(C, P, S.d[P.axis * kSmall + S.perm[f + P.nl]]) ? 0u : 1u);
+    if (c <= 32) {
+        const bool valid = lane < c;
+        const uint32_t j = valid ? S.perm[f + lane] : 0u;
+        const bool left = valid && goes_left_c(C, P, S.d[P.axis * kSmall + j]);
+        const unsigned m = __ballot_sync(0xffffffffu, left);
+        const uint32_t lpre = __popc(m & ((1u << lane) - 1u));
+        if (valid) {
+            if (lane < P.p && !left) S.F[f + (lane - lpre)] = (uint16_t)lane;
+            else if (lane >= P.p && left) S.G[f + (P.nl - lpre) - 1] = (uint16_t)lane;
+        }
+        __syncwarp();
+        if (valid) {
+            uint32_t dst;
+            if (lane < P.p) {
+                const uint32_t mm = lane - lpre + 1;
+                dst = left ? lane : (mm == 1 ? c : (uint32_t)S.G[f + mm - 2]) - 1;
+            } else {
+                dst = !left ? lane - 1 : (uint32_t)S.F[f + (P.nl - lpre) - 1];
+            }
+            S.perm[f + dst] = (uint16_t)j;
+        }
+        __syncwarp();
+    } else {
+        for (int pass = 0; pass < 2; ++pass) {
+            uint32_t run = 0;
+            for (uint32_t base = 0; base < c; base += 32) {
+                const uint32_t i = base + lane;
+                const bool valid = i < c;
+                const uint32_t j = valid ? S.perm[f + i] : 0u;
+                const bool left = valid && goes_left_c(C, P, S.d[P.axis * kSmall + j]);
+                const unsigned m = __ballot_sync(0xffffffffu, left);
+                const uint32_t lpre = run + __popc(m & ((1u << lane) - 1u));
+                if (valid) {
+                    if (pass == 0) {
+                        if (i < P.p && !left) S.F[f + (i - lpre)] = (uint16_t)i;
+                        else if (i >= P.p && left) S.G[f + (P.nl - lpre) - 1] = (uint16_t)i;
+                    } else {
+                        uint32_t dst;
+                        if (i < P.p) {
+                            const uint32_t mm = i - lpre + 1;
+                            dst = left ? i : (mm == 1 ? c : (uint32_t)S.G[f + mm - 2]) - 1;
+                        } else {
+                            dst = !left ? i - 1 : (uint32_t)S.F[f + (P.nl - lpre) - 1];
+                        }
+                        S.ptmp[f + dst] = (uint16_t)j;
+                    }
+                }
+                run += __popc(m);
+            }
+            __syncwarp();
+        }
+        for (uint32_t i = lane; i < c; i += 32) S.perm[f + i] = S.ptmp[f + i];
+        __syncwarp();
+    }
+    return P.children ? P.nl : 0u;
+}
+
+__global__ void __launch_bounds__(32 * kSmallWarps) k_small(Ctx C, uint32_t nsmall, uint32_t tcap) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
+    __shared__ uint32_t s_count[2], s_base, s_splits;
     SmallSmem S;
     S.d = reinterpret_cast<float*>(smem_raw);
     S.oidx = reinterpret_cast<uint32_t*>(S.d + 9 * kSmall);
-    S.perm = reinterpret_cast<uint16_t*>(S.oidx + kSmall);
+    S.task[0] = S.oidx + kSmall;
+    S.task[1] = S.task[0] + kSmall;
+    S.perm = reinterpret_cast<uint16_t*>(S.task[1] + kSmall);
     S.ptmp = S.perm + kSmall;
     S.F = S.ptmp + kSmall;
     S.G = S.F + kSmall;
     S.bins = reinterpret_cast<uint32_t*>(S.G + kSmall);
-    const uint32_t lane = threadIdx.x;
-    const uint32_t words = 3 * C.bins * kBinWords;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    uint32_t* bins = S.bins + warp * 3 * C.bins * kBinWords;
     for (uint32_t w = blockIdx.x; w < nsmall; w += gridDim.x) {
         const uint32_t R = C.small_list[w];
         const uint32_t gfirst = __float_as_uint(C.ta[R].w), count = __float_as_uint(C.tb[R].w);
-        const uint32_t depth0 = C.tdepth[R];
-        for (uint32_t i = lane; i < count; i += 32) {
-            const uint32_t t = C.idx[gfirst + i];
-            const float4 c = C.cen[t], mn = C.tmn[t], mx = C.tmx[t];
+        uint32_t dep = C.tdepth[R];
+        for (uint32_t i = t; i < count; i += 32 * kSmallWarps) {
+            const uint32_t id = C.idx[gfirst + i];
+            const float4 c = C.cen[id], mn = C.tmn[id], mx = C.tmx[id];
             S.d[0 * kSmall + i] = c.x;  S.d[1 * kSmall + i] = c.y;  S.d[2 * kSmall + i] = c.z;
             S.d[3 * kSmall + i] = mn.x; S.d[4 * kSmall + i] = mn.y; S.d[5 * kSmall + i] = mn.z;
             S.d[6 * kSmall + i] = mx.x; S.d[7 * kSmall + i] = mx.y; S.d[8 * kSmall + i] = mx.z;
-            S.oidx[i] = t;
+            S.oidx[i] = id;
             S.perm[i] = (uint16_t)i;
         }
-        uint32_t L0 = 0;
-        if (lane == 0) L0 = atomicAdd(&C.tcount[0], 2u * (count - 1));
-        L0 = __shfl_sync(0xffffffffu, L0, 0);
+        if (t == 0) {
+            s_base = atomicAdd(&C.tcount[0], 2u * (count - 1));
+            s_count[0] = 1u;
+            s_count[1] = 0u;
+            s_splits = 0u;
+            S.task[0][0] = 0u | (count << 8);
+        }
+        __syncthreads();
+        const uint32_t L0 = s_base;
         if ((uint64_t)L0 + 2ull * (count - 1) > tcap) {   // cannot happen for tcap = 2n + 2n / kSmall + 4
-            if (lane == 0) atomicOr(&C.tcount[3], 1u);
+            if (t == 0) atomicOr(&C.tcount[3], 1u);
+            __syncthreads();
             continue;
         }
-        __syncwarp();
-        uint32_t splits = 0, maxd = depth0, sp = 0;
-        uint32_t sX = 0, sf = 0, sc = 0, sd = 0;   // stack entry `lane`
-        uint32_t X = R, f = 0, c = count, dep = depth0;
-        for (;;) {
-            // node bounds, centroid bounds and first zero positions
-            float v[12];
-            uint32_t zp[6];
-            box_init(v);
-            zero_init(zp);
-            for (uint32_t i = lane; i < c; i += 32) {
-                const uint32_t j = S.perm[f + i];
-                float e[9];
-                for (int k = 0; k < 9; ++k) e[k] = S.d[k * kSmall + j];
-                v[0] = gmin(v[0], e[3]); v[1] = gmin(v[1], e[4]); v[2] = gmin(v[2], e[5]);
-                v[3] = gmax(v[3], e[6]); v[4] = gmax(v[4], e[7]); v[5] = gmax(v[5], e[8]);
-                v[6] = gmin(v[6], e[0]); v[7] = gmin(v[7], e[1]); v[8] = gmin(v[8], e[2]);
-                v[9] = gmax(v[9], e[0]); v[10] = gmax(v[10], e[1]); v[11] = gmax(v[11], e[2]);
-                for (int k = 0; k < 6; ++k)
-                    if (e[3 + k] == 0.0f && zp[k] == kNone) zp[k] = i;
-            }
-            box_warp_reduce(v);
-            zero_warp_reduce(zp);
-            for (int k = 0; k < 6; ++k)
-                if (v[k] == 0.0f && zp[k] != kNone) v[k] = S.d[(3 + k) * kSmall + S.perm[f + zp[k]]];
-            if (lane == 0) {
-                C.ta[X] = make_float4(v[0], v[1], v[2], __uint_as_float(gfirst + f));
-                C.tb[X] = make_float4(v[3], v[4], v[5], __uint_as_float(c));
-                C.tleft[X] = kNone;
-                C.tdepth[X] = dep;
-            }
-            bool deg[3];
-            float lo[3], scale[3];
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = v[6 + a];
-                deg[a] = v[6 + a] == v[9 + a];
-                scale[a] = deg[a] ? 0.0f : (float)C.bins / (v[9 + a] - v[6 + a]);
-            }
-            bins_reset(S.bins, words, lane, 32);
-            __syncwarp();
-            for (uint32_t i = lane; i < c; i += 32) {
-                const uint32_t j = S.perm[f + i];
-                for (uint32_t a = 0; a < 3; ++a) {
-                    if (deg[a]) continue;
-                    int32_t bin = (int32_t)((S.d[a * kSmall + j] - lo[a]) * scale[a]);
-                    if ((int32_t)C.bins - 1 < bin) bin = (int32_t)C.bins - 1;
-                    uint32_t* e = S.bins + (a * C.bins + (uint32_t)bin) * kBinWords;
-                    atomicAdd(&e[0], 1u);
-                    atomicMin(&e[1], fenc(S.d[3 * kSmall + j]));
-                    atomicMin(&e[2], fenc(S.d[4 * kSmall + j]));
-                    atomicMin(&e[3], fenc(S.d[5 * kSmall + j]));
-                    atomicMax(&e[4], fenc(S.d[6 * kSmall + j]));
-                    atomicMax(&e[5], fenc(S.d[7 * kSmall + j]));
-                    atomicMax(&e[6], fenc(S.d[8 * kSmall + j]));
+        uint32_t cur = 0;
+        for (uint32_t nodes = 1; nodes > 0;) {
+            for (uint32_t q = warp; q < nodes; q += kSmallWarps) {
+                const uint32_t task = S.task[cur][q];
+                const uint32_t f = task & 0xFFu, c = (task >> 8) & 0xFFu, k = task >> 16;
+                const uint32_t X = k == 0u ? R : L0 + k - 1u;
+                const uint32_t nl = small_node(C, S, bins, X, gfirst, f, c, dep, lane);
+                if (nl && lane == 0) {
+                    const uint32_t kl = 2u * atomicAdd(&s_splits, 1u);
+                    C.tleft[X] = L0 + kl;
+                    const uint32_t at = atomicAdd(&s_count[cur ^ 1], 2u);
+                    S.task[cur ^ 1][at] = f | (nl << 8) | ((kl + 1u) << 16);
+                    S.task[cur ^ 1][at + 1] = (f + nl) | ((c - nl) << 8) | ((kl + 2u) << 16);
                 }
-            }
-            __syncwarp();
-            Plan P = make_plan_warp(C, S.bins, c, v, v + 3, v + 6, v + 9, lane);
-            if (P.partition && P.nl < c)
-                P.p = P.nl + (goes_left_c(C, P, S.d[P.axis * kSmall + S.perm[f + P.nl]]) ? 0u : 1u);
-            __syncwarp();
-            if (P.partition) {
-                // the closed form of the two-pointer partition (see the file head),
-                // positions relative to the node's first position f
-                for (int pass = 0; pass < 2; ++pass) {
-                    uint32_t run = 0;
-                    for (uint32_t base = 0; base < c; base += 32) {
-                        const uint32_t i = base + lane;
-                        const bool valid = i < c;
-                        const uint32_t j = valid ? S.perm[f + i] : 0u;
-                        const bool left = valid && goes_left_c(C, P, S.d[P.axis * kSmall + j]);
-                        const unsigned m = __ballot_sync(0xffffffffu, left);
-                        const uint32_t lpre = run + __popc(m & ((1u << lane) - 1u));
-                        if (valid) {
-                            if (pass == 0) {
-                                if (i < P.p && !left) S.F[f + (i - lpre)] = (uint16_t)i;
-                                else if (i >= P.p && left) S.G[f + (P.nl - lpre) - 1] = (uint16_t)i;
-                            } else {
-                                uint32_t dst;
-                                if (i < P.p) {
-                                    const uint32_t mm = i - lpre + 1;
-                                    dst = left ? i : (mm == 1 ? c : (uint32_t)S.G[f + mm - 2]) - 1;
-                                } else {
-                                    dst = !left ? i - 1 : (uint32_t)S.F[f + (P.nl - lpre) - 1];
-                                }
-                                S.ptmp[f + dst] = (uint16_t)j;
-                            }
-                        }
-                        run += __popc(m);
-                    }
-                    __syncwarp();
-                }
-                for (uint32_t i = lane; i < c; i += 32) S.perm[f + i] = S.ptmp[f + i];
                 __syncwarp();
             }
-            if (P.children) {
-                const uint32_t L = L0 + 2 * splits++;
-                if (lane == 0) C.tleft[X] = L;
-                const uint32_t nl = P.nl, nr = c - P.nl;
-                maxd = max(maxd, dep + 1);
-                // descend into the smaller child, push the larger
-                const bool go_left = nl <= nr;
-                if (lane == sp) {
-                    sX = go_left ? L + 1 : L;
-                    sf = go_left ? f + nl : f;
-                    sc = go_left ? nr : nl;
-                    sd = dep + 1;
-                }
-                ++sp;
-                X = go_left ? L : L + 1;
-                f = go_left ? f : f + nl;
-                c = go_left ? nl : nr;
-                dep = dep + 1;
-                continue;
-            }
-            if (sp == 0) break;
-            --sp;
-            X = __shfl_sync(0xffffffffu, sX, sp);
-            f = __shfl_sync(0xffffffffu, sf, sp);
-            c = __shfl_sync(0xffffffffu, sc, sp);
-            dep = __shfl_sync(0xffffffffu, sd, sp);
+            __syncthreads();
+            nodes = s_count[cur ^ 1];
+            if (t == 0) s_count[cur] = 0u;   // read by no one now, filled after the next barrier
+            __syncthreads();
+            cur ^= 1u;
+            if (nodes) ++dep;
         }
-        for (uint32_t i = lane; i < count; i += 32) C.idx[gfirst + i] = S.oidx[S.perm[i]];
-        if (lane == 0) atomicMax(&C.tcount[1], maxd);
-        __syncwarp();
+        for (uint32_t i = t; i < count; i += 32 * kSmallWarps) C.idx[gfirst + i] = S.oidx[S.perm[i]];
+        if (t == 0) atomicMax(&C.tcount[1], dep);
+        __syncthreads();
     }
 }
 
@@ -1118,7 +1164,7 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
         k_chunk_scan<<<1, 1024, 0, st>>>(C, Lv);
         k_bins_reset<<<blocks_for((uint64_t)nslots * 3 * B * kBinWords, 256), 256, 0, st>>>(C, Lv);
         k_bin_chunks<<<grid, kChunkThreads, 0, st>>>(C, Lv);
-        k_plan<<<sgrid, 128, 0, st>>>(C, Lv);
+        k_plan<<<(nslots + 3) / 4, 128, 0, st>>>(C, Lv);
         k_part_count<<<grid, kChunkThreads, 0, st>>>(C, Lv);
         k_part_slot_scan<<<sgrid, 128, 0, st>>>(C, Lv);
         k_part_pass<false><<<grid, kChunkThreads, 0, st>>>(C, Lv);
@@ -1139,7 +1185,7 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
         BVH_CUDA(cudaMemsetAsync(C.tdepth + counts[0], 0xFF, 4ull * (tcap - counts[0]), st));
         const size_t smem = small_smem_bytes(B);
         BVH_CUDA(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_small<<<counts[2], 32, smem, st>>>(C, counts[2], (uint32_t)tcap);
+        k_small<<<counts[2], 32 * kSmallWarps, smem, st>>>(C, counts[2], (uint32_t)tcap);
         BVH_CUDA(cudaGetLastError());
     }
     BVH_CUDA(cudaMemcpyAsync(counts, C.tcount, 16, cudaMemcpyDeviceToHost, st));
