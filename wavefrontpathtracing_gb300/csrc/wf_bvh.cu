@@ -29,9 +29,11 @@
 //    2 + 2 * (pre-order rank of X among internal nodes).
 //
 // Phases: nodes with more than kSmall triangles are processed level by level
-// by many CTAs (chunked binning into shared-memory bins, chunked scans for the
-// partition); subtrees of at most kSmall triangles are built by one warp each,
-// entirely in shared memory.  The host side makes one scratch allocation,
+// by the whole grid of one cooperative launch (chunked binning into
+// shared-memory bins, side bits and chunked scans for the partition); subtrees
+// of at most kSmall triangles are built by one CTA each, entirely in shared
+// memory; the renumbering climbs from the leaves once and from every node once.
+// Nothing is read back before the tree stands.  The host side makes one scratch allocation,
 // gathers the positions on several threads and writes the blob straight into
 // the caller's buffer when it fits.
 #include <algorithm>
@@ -48,8 +50,9 @@ namespace wf {
 namespace {
 
 constexpr uint32_t kMaxBins = 64;
-constexpr uint32_t kChunk = 4096;      // positions per CTA in the large-node phase
+constexpr uint32_t kChunk = 1024;      // positions a block of the large-node phase takes at a time: 32 words of side bits
 constexpr uint32_t kChunkThreads = 256;
+static_assert(kChunk == 1024 && kChunkThreads == 256, "a warp holds four of a chunk's 32 words");
 #ifndef WF_BVH_SMALL
 #define WF_BVH_SMALL 128
 #endif
@@ -82,15 +85,16 @@ struct Ctx {
     float4* cen;             // centroid
     float4* tmn;             // triangle min corner
     float4* tmx;             // triangle max corner
-    uint32_t* idx;           // current index permutation
-    uint32_t* idx_tmp;       // partition target
+    uint32_t* idx[2];        // index permutation: a node at depth d has its range in idx[d & 1]; the leaves'
+                             // ranges end in idx[0]
     uint32_t* F;             // per-position scratch: front right-goers by rank
     uint32_t* G;             // per-position scratch: back left-goers by rank
     float4* ta;              // temporary nodes {min xyz, first}
     float4* tb;              //                 {max xyz, count}
     uint32_t* tleft;         // left child (kNone for leaves); right child = left + 1
+    uint32_t* tparent;
     uint32_t* tdepth;
-    uint32_t* tcount;        // [0] nodes allocated, [1] maximum depth, [2] small roots, [3] error
+    uint32_t* tcount;        // [0] nodes allocated, [1] internal nodes, [2] small roots, [3] error
     uint32_t* small_list;
 };
 
@@ -267,25 +271,7 @@ __device__ __forceinline__ void partition_rank(const Ctx& C, const Plan& P, uint
     }
 }
 
-// ---------------------------------------------------------------- preparation
-__global__ void k_prep(Ctx C) {
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < C.n; t += stride) {
-        const float* p = C.pos + 9ull * t;
-        float c[3], mn[3], mx[3];
-        for (int a = 0; a < 3; ++a) {
-            float p0 = p[a], p1 = p[3 + a], p2 = p[6 + a];
-            c[a] = ((p0 + p1) + p2) * 0.3333f;
-            mn[a] = gmin(gmin(p0, p1), p2);
-            mx[a] = gmax(gmax(p0, p1), p2);
-        }
-        C.cen[t] = make_float4(c[0], c[1], c[2], 0.0f);
-        C.tmn[t] = make_float4(mn[0], mn[1], mn[2], 0.0f);
-        C.tmx[t] = make_float4(mx[0], mx[1], mx[2], 0.0f);
-        C.idx[t] = t;
-    }
-}
-
+// ---------------------------------------------------------------- bounds
 __device__ __forceinline__ void box_init(float* v) {
     for (int k = 0; k < 3; ++k) { v[k] = FLT_MAX; v[3 + k] = -FLT_MAX; v[6 + k] = FLT_MAX; v[9 + k] = -FLT_MAX; }
 }
@@ -313,115 +299,44 @@ __device__ __forceinline__ void zero_add(uint32_t* zp, const Ctx& C, uint32_t t,
     const float4 mn = C.tmn[t], mx = C.tmx[t];
     const float v[6] = {mn.x, mn.y, mn.z, mx.x, mx.y, mx.z};
     for (int k = 0; k < 6; ++k)
-        if (v[k] == 0.0f && zp[k] == kNone) zp[k] = position;
+        if (v[k] == 0.0f) zp[k] = min(zp[k], position);   // positions come in any order
 }
-__device__ __forceinline__ void zero_warp_reduce(uint32_t* zp) {
-    for (int off = 16; off > 0; off >>= 1)
-        for (int k = 0; k < 6; ++k) zp[k] = min(zp[k], __shfl_xor_sync(0xffffffffu, zp[k], off));
-}
-__device__ __forceinline__ void zero_fix(const Ctx& C, float* v, const uint32_t* zp) {
+__device__ __forceinline__ void zero_fix(const Ctx& C, const uint32_t* idx, float* v, const uint32_t* zp) {
     for (int k = 0; k < 6; ++k)
-        if (v[k] == 0.0f && zp[k] != kNone) v[k] = tri_comp(C, C.idx[zp[k]], k);
+        if (v[k] == 0.0f && zp[k] != kNone) v[k] = tri_comp(C, idx[zp[k]], k);
 }
-
-__device__ __forceinline__ void box_warp_reduce(float* v) {
-    for (int off = 16; off > 0; off >>= 1) {
-        for (int k = 0; k < 12; ++k) {
-            float o = __shfl_xor_sync(0xffffffffu, v[k], off);
-            v[k] = ((k % 6) < 3) ? gmin(v[k], o) : gmax(v[k], o);
+// Warp-wide bounds from per-lane folds: v = node min / max, centroid min / max.
+__device__ __forceinline__ void box_warp_redux(float* v) {
+#pragma unroll
+    for (int k = 0; k < 12; ++k)
+        v[k] = fdec((k % 6) < 3 ? __reduce_min_sync(0xffffffffu, fenc(v[k])) : __reduce_max_sync(0xffffffffu, fenc(v[k])));
+}
+// A warp's folds into a box's keys (shared or global memory).  Only a warp whose
+// own bound is zero can hold the first zero of a zero bound.
+__device__ __forceinline__ void box_warp_atomic(uint32_t* keys, float* v, const uint32_t* zp, uint32_t lane) {
+    box_warp_redux(v);
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        if (lane == (uint32_t)k) {
+            if ((k % 6) < 3) atomicMin(&keys[k], fenc(v[k]));
+            else atomicMax(&keys[k], fenc(v[k]));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        if (v[k] == 0.0f) {
+            const uint32_t z = __reduce_min_sync(0xffffffffu, zp[k]);
+            if (lane == 0 && z != kNone) atomicMin(&keys[12 + k], z);
         }
     }
 }
-__device__ __forceinline__ void box_atomic(uint32_t* keys, const float* v, const uint32_t* zp) {
-    for (int k = 0; k < 12; ++k) {
-        if ((k % 6) < 3) atomicMin(&keys[k], fenc(v[k]));
-        else atomicMax(&keys[k], fenc(v[k]));
-    }
-    for (int k = 0; k < 6; ++k)
-        if (zp[k] != kNone) atomicMin(&keys[12 + k], zp[k]);
+__device__ __forceinline__ void box_merge(uint32_t* to, uint32_t key, uint32_t k) {
+    if (k >= 12 || (k % 6) < 3) atomicMin(&to[k], key);
+    else atomicMax(&to[k], key);
 }
 
 __device__ __forceinline__ uint32_t key_init(uint32_t k) {
     return k >= 12 ? kNone : (((k % 6) < 3) ? fenc(FLT_MAX) : fenc(-FLT_MAX));
-}
-
-// Bounds of the root (all positions) into slot keys.
-__global__ void k_root_bounds(Ctx C, uint32_t* keys) {
-    float v[12];
-    uint32_t zp[6];
-    box_init(v);
-    zero_init(zp);
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < C.n; i += stride) {
-        const uint32_t t = C.idx[i];
-        box_add(v, C, t);
-        zero_add(zp, C, t, i);
-    }
-    box_warp_reduce(v);
-    zero_warp_reduce(zp);
-    if ((threadIdx.x & 31) == 0) box_atomic(keys, v, zp);
-}
-
-__global__ void k_keys_init(uint32_t* keys, uint32_t count_words) {
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count_words; i += stride)
-        keys[i] = key_init(i % kBoxWords);
-}
-
-// ---------------------------------------------------------------- large-node phase
-struct Level {
-    uint32_t nslots;
-    const uint32_t* slot_tmp;   // tmp node id per slot
-    const uint32_t* slot_box;   // 12 keys per slot
-    uint32_t* bins;             // slot x 3 x B x 7
-    uint32_t* chunk_off;        // exclusive prefix of chunks per slot, [nslots] = total
-    uint32_t* chunk_l;          // left-goers per chunk, then their per-slot exclusive prefix
-    Plan* plan;                 // per slot
-    uint32_t* child_slot;       // per slot x 2: next-level slot or kNone
-    uint32_t* next_tmp;
-    uint32_t* next_box;
-    uint32_t* next_count;
-};
-
-__global__ void k_chunk_scan(Ctx C, Level Lv) {
-    // one block of 1024 threads; each thread owns a contiguous run of slots
-    __shared__ uint32_t part[1024];
-    const uint32_t per = (Lv.nslots + 1023) / 1024;
-    const uint32_t s0 = threadIdx.x * per, s1 = min(Lv.nslots, s0 + per);
-    uint32_t sum = 0;
-    for (uint32_t s = s0; s < s1; ++s) sum += (__float_as_uint(C.tb[Lv.slot_tmp[s]].w) + kChunk - 1) / kChunk;
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    for (uint32_t off = 1; off < 1024; off <<= 1) {
-        uint32_t v = threadIdx.x >= off ? part[threadIdx.x - off] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    uint32_t run = part[threadIdx.x] - sum;
-    for (uint32_t s = s0; s < s1; ++s) {
-        Lv.chunk_off[s] = run;
-        run += (__float_as_uint(C.tb[Lv.slot_tmp[s]].w) + kChunk - 1) / kChunk;
-    }
-    if (threadIdx.x == 1023) Lv.chunk_off[Lv.nslots] = part[1023];
-}
-
-// Maps a block to (slot, first, count, local range); false if past the end.
-__device__ __forceinline__ bool chunk_of(const Ctx& C, const Level& Lv, uint32_t b, uint32_t& slot, uint32_t& first,
-                                         uint32_t& count, uint32_t& i0, uint32_t& i1) {
-    if (b >= Lv.chunk_off[Lv.nslots]) return false;
-    uint32_t lo = 0, hi = Lv.nslots - 1;
-    while (lo < hi) {
-        uint32_t mid = (lo + hi + 1) >> 1;
-        if (Lv.chunk_off[mid] <= b) lo = mid; else hi = mid - 1;
-    }
-    slot = lo;
-    const uint32_t t = Lv.slot_tmp[slot];
-    first = __float_as_uint(C.ta[t].w);
-    count = __float_as_uint(C.tb[t].w);
-    i0 = (b - Lv.chunk_off[slot]) * kChunk;
-    i1 = min(count, i0 + kChunk);
-    return true;
 }
 
 __device__ __forceinline__ void bins_reset(uint32_t* sb, uint32_t words, uint32_t tid, uint32_t nthreads) {
@@ -429,6 +344,134 @@ __device__ __forceinline__ void bins_reset(uint32_t* sb, uint32_t words, uint32_
         uint32_t k = w % kBinWords;
         sb[w] = k == 0 ? 0u : (k < 4 ? fenc(FLT_MAX) : fenc(-FLT_MAX));
     }
+}
+
+// ---------------------------------------------------------------- large-node phase
+// Nodes of more than kSmall triangles, level by level, in one cooperative
+// launch: each step of a level (bins, plans, sides, ranks, move) is a phase of
+// the grid, with a grid-wide barrier after it.  Bound by the barriers and the
+// latency of a step where a level has few chunks, by the partition's scattered
+// reads (centroid, box) where it has many.  A launch per step (12 per level),
+// with the level's node count read back by the host, took about 100 us per
+// level however few triangles it had; us per wf_bvh_build, so / in one launch,
+// with the renumbering below: 80 triangles 296 / 190, 1,280: 672 / 356, 20,480:
+// 1,634 / 851, 100,820: 2,684 / 1,560, 499,280: 7,423 / 6,180 (4.8 ms of it the
+// host's copies).
+//
+// A slot is a node of the level, a chunk kChunk consecutive positions of one
+// slot; a block takes chunks in turn.  Slots and chunks of the next level are
+// numbered as their parents are planned (their order changes nothing).
+struct Large {
+    uint32_t* slot_tmp[2];      // by level parity: node id per slot
+    uint32_t* slot_box[2];      // kBoxWords keys per slot
+    uint32_t* slot_done[2];     // 1: nothing left but to end in idx[0]
+    uint32_t* slot_chunk[2];    // first chunk per slot
+    uint32_t* chunk_slot[2];
+    Plan* plan;                 // per slot
+    uint32_t* child_slot;       // per slot x 2: next-level slot or kNone
+    uint32_t* bins;             // slot x 3 x B x 7
+    uint32_t* chunk_l;          // left-goers per chunk
+    uint32_t* side;             // 32 words per chunk: bit = the position's triangle goes left
+    uint32_t* cnt;              // [0..1] slots, [2..3] chunks by parity, [4] arrivals at the barrier
+};
+
+// Everything a build starts from (one block): the root as node 0 and, when it
+// is large, as the first level's slot.
+__global__ void k_init(Ctx C, Large G) {
+    const uint32_t t = threadIdx.x, nch = (C.n + kChunk - 1) / kChunk;
+    const bool large = C.n > kSmall;
+    if (t == 0) {
+        C.ta[0] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(0u));
+        C.tb[0] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(C.n));
+        C.tleft[0] = kNone;
+        C.tparent[0] = 0u;
+        C.tdepth[0] = 0u;
+        C.tcount[0] = 1u; C.tcount[1] = 0u; C.tcount[2] = large ? 0u : 1u; C.tcount[3] = 0u;
+        C.small_list[0] = 0u;
+        G.slot_tmp[0][0] = 0u; G.slot_done[0][0] = 0u; G.slot_chunk[0][0] = 0u;
+        G.cnt[0] = large ? 1u : 0u; G.cnt[1] = 0u; G.cnt[2] = large ? nch : 0u; G.cnt[3] = 0u; G.cnt[4] = 0u;
+    }
+    if (t < kBoxWords) G.slot_box[0][t] = key_init(t);
+    if (!large) return;
+    for (uint32_t k = t; k < nch; k += blockDim.x) G.chunk_slot[0][k] = 0u;
+    bins_reset(G.bins, 3 * C.bins * kBinWords, t, blockDim.x);
+}
+
+// Centroid and box per triangle, and the root's bounds.
+__global__ void __launch_bounds__(256) k_prep(Ctx C, uint32_t* root_box) {
+    __shared__ uint32_t s_box[kBoxWords];
+    if (threadIdx.x < kBoxWords) s_box[threadIdx.x] = key_init(threadIdx.x);
+    __syncthreads();
+    float v[12];
+    uint32_t zp[6];
+    box_init(v);
+    zero_init(zp);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < C.n; t += stride) {
+        const float* p = C.pos + 9ull * t;
+        float c[3], mn[3], mx[3];
+        for (int a = 0; a < 3; ++a) {
+            float p0 = p[a], p1 = p[3 + a], p2 = p[6 + a];
+            c[a] = ((p0 + p1) + p2) * 0.3333f;
+            mn[a] = gmin(gmin(p0, p1), p2);
+            mx[a] = gmax(gmax(p0, p1), p2);
+            v[a] = fminf(v[a], mn[a]);
+            v[3 + a] = fmaxf(v[3 + a], mx[a]);
+            v[6 + a] = fminf(v[6 + a], c[a]);
+            v[9 + a] = fmaxf(v[9 + a], c[a]);
+            if (mn[a] == 0.0f && zp[a] == kNone) zp[a] = t;
+            if (mx[a] == 0.0f && zp[3 + a] == kNone) zp[3 + a] = t;
+        }
+        C.cen[t] = make_float4(c[0], c[1], c[2], 0.0f);
+        C.tmn[t] = make_float4(mn[0], mn[1], mn[2], 0.0f);
+        C.tmx[t] = make_float4(mx[0], mx[1], mx[2], 0.0f);
+        C.idx[0][t] = t;
+    }
+    if (!root_box) return;
+    box_warp_atomic(s_box, v, zp, threadIdx.x & 31u);
+    __syncthreads();
+    if (threadIdx.x < kBoxWords) box_merge(root_box, s_box[threadIdx.x], threadIdx.x);
+}
+
+// All blocks of the (cooperative) grid; false once it waited too long, which a
+// correct run never does: the build then ends with an error.
+__device__ bool grid_barrier(uint32_t* arrivals, uint32_t* error, uint32_t& round) {
+    __shared__ uint32_t s_ok;
+    __syncthreads();
+    ++round;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(arrivals, 1u);
+        const uint32_t target = round * gridDim.x;
+        uint32_t ok = 1u, spins = 0;
+        while ((int32_t)(*(volatile uint32_t*)arrivals - target) < 0) {
+            if (++spins > (1u << 22) || *(volatile uint32_t*)error) {
+                atomicOr(error, 2u);
+                ok = 0u;
+                break;
+            }
+            __nanosleep(32);
+        }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0u;
+}
+
+// A chunk: its slot and positions [i0, i1) of the slot's [first, first + count).
+struct Chunk {
+    uint32_t slot, first, count, i0, i1;
+};
+__device__ __forceinline__ Chunk chunk_of(const Ctx& C, const Large& G, uint32_t cur, uint32_t b) {
+    Chunk k;
+    k.slot = G.chunk_slot[cur][b];
+    const uint32_t t = G.slot_tmp[cur][k.slot];
+    k.first = __float_as_uint(C.ta[t].w);
+    k.count = __float_as_uint(C.tb[t].w);
+    k.i0 = (b - G.slot_chunk[cur][k.slot]) * kChunk;
+    k.i1 = min(k.count, k.i0 + kChunk);
+    return k;
 }
 
 __device__ __forceinline__ void bin_element(const Ctx& C, uint32_t* sb, uint32_t t, const bool* deg, const float* lo,
@@ -445,20 +488,12 @@ __device__ __forceinline__ void bin_element(const Ctx& C, uint32_t* sb, uint32_t
     }
 }
 
-__global__ void k_bins_reset(Ctx C, Level Lv) {
-    const uint32_t words = Lv.nslots * 3 * C.bins * kBinWords;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += stride) {
-        uint32_t k = w % kBinWords;
-        Lv.bins[w] = k == 0 ? 0u : (k < 4 ? fenc(FLT_MAX) : fenc(-FLT_MAX));
-    }
-}
-
-__global__ void __launch_bounds__(kChunkThreads) k_bin_chunks(Ctx C, Level Lv) {
-    __shared__ uint32_t sb[3 * kMaxBins * kBinWords];
-    uint32_t slot, first, count, i0, i1;
-    if (!chunk_of(C, Lv, blockIdx.x, slot, first, count, i0, i1)) return;
-    const uint32_t* key = Lv.slot_box + kBoxWords * slot;
+// A chunk's bins, summed in shared memory and merged into its slot's.
+__device__ __forceinline__ void bin_chunk(const Ctx& C, const Large& G, uint32_t cur, const uint32_t* idx, uint32_t b,
+                                          uint32_t* sb) {
+    const Chunk k = chunk_of(C, G, cur, b);
+    if (G.slot_done[cur][k.slot]) return;
+    const uint32_t* key = G.slot_box[cur] + kBoxWords * k.slot;
     bool deg[3];
     float lo[3], scale[3];
     for (int a = 0; a < 3; ++a) {
@@ -470,191 +505,216 @@ __global__ void __launch_bounds__(kChunkThreads) k_bin_chunks(Ctx C, Level Lv) {
     const uint32_t words = 3 * C.bins * kBinWords;
     bins_reset(sb, words, threadIdx.x, blockDim.x);
     __syncthreads();
-    for (uint32_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) bin_element(C, sb, C.idx[first + i], deg, lo, scale);
+    for (uint32_t i = k.i0 + threadIdx.x; i < k.i1; i += blockDim.x) bin_element(C, sb, idx[k.first + i], deg, lo, scale);
     __syncthreads();
-    uint32_t* gb = Lv.bins + (size_t)slot * words;
+    uint32_t* gb = G.bins + (size_t)k.slot * words;
     for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) {
-        const uint32_t k = w % kBinWords;
-        if (deg[w / (C.bins * kBinWords)]) continue;
-        if (k == 0) { if (sb[w]) atomicAdd(&gb[w], sb[w]); }
-        else if (k < 4) atomicMin(&gb[w], sb[w]);
+        const uint32_t q = w % kBinWords, e = w - q;
+        if (sb[e] == 0u) continue;   // an empty bin (or a degenerate axis)
+        if (q == 0) atomicAdd(&gb[w], sb[w]);
+        else if (q < 4) atomicMin(&gb[w], sb[w]);
         else atomicMax(&gb[w], sb[w]);
     }
-}
-
-// A warp per slot.
-__global__ void k_plan(Ctx C, Level Lv) {
-    const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (s >= Lv.nslots) return;
-    const uint32_t t = Lv.slot_tmp[s];
-    const uint32_t* key = Lv.slot_box + kBoxWords * s;
-    float box[6], cmn[3], cmx[3];
-    for (int a = 0; a < 3; ++a) {
-        box[a] = fdec(key[a]); box[3 + a] = fdec(key[3 + a]);
-        cmn[a] = fdec(key[6 + a]); cmx[a] = fdec(key[9 + a]);
-    }
-    zero_fix(C, box, key + 12);
-    const float* nmn = box;
-    const float* nmx = box + 3;
-    const uint32_t first = __float_as_uint(C.ta[t].w), count = __float_as_uint(C.tb[t].w);
-    uint32_t axis, pos, nl;
-    const float cost = warp_sweep(Lv.bins + (size_t)s * 3 * C.bins * kBinWords, C.bins, cmn, cmx, lane, axis, pos, nl);
-    Plan P = plan_from(C, cost, axis, pos, nl, count, nmn, nmx, cmn, cmx);
-    // the element at position nl decides where the front part ends
-    if (P.partition && P.nl < count) P.p = P.nl + (goes_left(C, P, C.idx[first + P.nl]) ? 0u : 1u);
-    if (lane == 0) {
-        C.ta[t] = make_float4(nmn[0], nmn[1], nmn[2], __uint_as_float(first));
-        C.tb[t] = make_float4(nmx[0], nmx[1], nmx[2], __uint_as_float(count));
-        Lv.plan[s] = P;
-    }
-}
-
-// Block-wide exclusive prefix of a flag (blockDim.x <= 1024); returns the prefix
-// and writes the block total to *total.
-__device__ __forceinline__ uint32_t block_prefix(bool flag, uint32_t* warp_sums, uint32_t* total) {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const unsigned m = __ballot_sync(0xffffffffu, flag);
-    const uint32_t in_warp = __popc(m & ((1u << lane) - 1u));
-    if (lane == 0) warp_sums[warp] = __popc(m);
     __syncthreads();
-    uint32_t before = 0, all = 0;
-    for (uint32_t w = 0; w < nw; ++w) {
-        if (w < warp) before += warp_sums[w];
-        all += warp_sums[w];
-    }
-    __syncthreads();
-    *total = all;
-    return before + in_warp;
 }
 
-__global__ void __launch_bounds__(kChunkThreads) k_part_count(Ctx C, Level Lv) {
-    __shared__ uint32_t ws[32];
-    uint32_t slot, first, count, i0, i1;
-    if (!chunk_of(C, Lv, blockIdx.x, slot, first, count, i0, i1)) return;
-    const Plan P = Lv.plan[slot];
-    if (!P.partition) return;
-    uint32_t sum = 0;
-    for (uint32_t base = i0; base < i1; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool left = i < i1 && goes_left(C, P, C.idx[first + i]);
-        uint32_t tot;
-        block_prefix(left, ws, &tot);
-        sum += tot;
-    }
-    if (threadIdx.x == 0) Lv.chunk_l[blockIdx.x] = sum;
-}
-
-__global__ void k_part_slot_scan(Ctx C, Level Lv) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= Lv.nslots || !Lv.plan[s].partition) return;
-    uint32_t run = 0;
-    for (uint32_t b = Lv.chunk_off[s]; b < Lv.chunk_off[s + 1]; ++b) {
-        uint32_t v = Lv.chunk_l[b];
-        Lv.chunk_l[b] = run;
-        run += v;
-    }
-}
-
-template <bool MOVE>
-__global__ void __launch_bounds__(kChunkThreads) k_part_pass(Ctx C, Level Lv) {
-    __shared__ uint32_t ws[32];
-    uint32_t slot, first, count, i0, i1;
-    if (!chunk_of(C, Lv, blockIdx.x, slot, first, count, i0, i1)) return;
-    const Plan P = Lv.plan[slot];
-    if (!P.partition) return;
-    uint32_t run = Lv.chunk_l[blockIdx.x];
-    for (uint32_t base = i0; base < i1; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool valid = i < i1;
-        const uint32_t t = valid ? C.idx[first + i] : 0u;
-        const bool left = valid && goes_left(C, P, t);
-        uint32_t tot;
-        const uint32_t lpre = run + block_prefix(left, ws, &tot);
-        if (valid) {
-            if (MOVE) C.idx_tmp[first + partition_dst(C, P, first, count, i, left, lpre)] = t;
-            else partition_rank(C, P, first, i, left, lpre);
-        }
-        run += tot;
-    }
-}
-
-__global__ void __launch_bounds__(kChunkThreads) k_part_copy(Ctx C, Level Lv) {
-    uint32_t slot, first, count, i0, i1;
-    if (!chunk_of(C, Lv, blockIdx.x, slot, first, count, i0, i1)) return;
-    if (!Lv.plan[slot].partition) return;
-    for (uint32_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) C.idx[first + i] = C.idx_tmp[first + i];
-}
-
-__device__ __forceinline__ void new_children(const Ctx& C, uint32_t X, uint32_t first, uint32_t count, uint32_t nl,
-                                             uint32_t& L) {
-    L = atomicAdd(&C.tcount[0], 2u);
-    const uint32_t d = C.tdepth[X] + 1;
-    C.ta[L] = make_float4(0, 0, 0, __uint_as_float(first));
-    C.tb[L] = make_float4(0, 0, 0, __uint_as_float(nl));
-    C.ta[L + 1] = make_float4(0, 0, 0, __uint_as_float(first + nl));
-    C.tb[L + 1] = make_float4(0, 0, 0, __uint_as_float(count - nl));
-    C.tleft[L] = kNone;
-    C.tleft[L + 1] = kNone;
-    C.tdepth[L] = d;
-    C.tdepth[L + 1] = d;
-    C.tleft[X] = L;
-    atomicMax(&C.tcount[1], d);
-}
-
-__global__ void k_children(Ctx C, Level Lv) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= Lv.nslots) return;
-    const Plan P = Lv.plan[s];
-    Lv.child_slot[2 * s] = kNone;
-    Lv.child_slot[2 * s + 1] = kNone;
-    if (!P.children) return;
-    const uint32_t X = Lv.slot_tmp[s];
+// One warp: a slot's plan, its children and, where they are large, their slots
+// and chunks at the next level.
+__device__ __forceinline__ void plan_slot(const Ctx& C, const Large& G, uint32_t cur, const uint32_t* idx, uint32_t s,
+                                          uint32_t lane) {
+    const uint32_t nxt = cur ^ 1u, X = G.slot_tmp[cur][s];
     const uint32_t first = __float_as_uint(C.ta[X].w), count = __float_as_uint(C.tb[X].w);
-    uint32_t L;
-    new_children(C, X, first, count, P.nl, L);
-    const uint32_t cnt[2] = {P.nl, count - P.nl};
-    for (uint32_t side = 0; side < 2; ++side) {
-        if (cnt[side] > kSmall) {
-            const uint32_t j = atomicAdd(Lv.next_count, 1u);
-            Lv.next_tmp[j] = L + side;
-            uint32_t* key = Lv.next_box + kBoxWords * j;
-            for (uint32_t k = 0; k < kBoxWords; ++k) key[k] = key_init(k);
-            Lv.child_slot[2 * s + side] = j;
-        } else {
-            C.small_list[atomicAdd(&C.tcount[2], 1u)] = L + side;
+    Plan P{};
+    uint32_t cs[2] = {kNone, kNone};
+    // slot j of the next level: node Y with c triangles
+    auto add_slot = [&](uint32_t Y, uint32_t c, uint32_t done) -> uint32_t {
+        const uint32_t nch = (c + kChunk - 1) / kChunk;
+        uint32_t j = 0, base = 0;
+        if (lane == 0) {
+            j = atomicAdd(&G.cnt[nxt], 1u);
+            base = atomicAdd(&G.cnt[2 + nxt], nch);
+            G.slot_tmp[nxt][j] = Y;
+            G.slot_done[nxt][j] = done;
+            G.slot_chunk[nxt][j] = base;
         }
+        j = __shfl_sync(0xffffffffu, j, 0);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (lane < kBoxWords) G.slot_box[nxt][kBoxWords * j + lane] = key_init(lane);
+        for (uint32_t q = lane; q < nch; q += 32) G.chunk_slot[nxt][base + q] = j;
+        return j;
+    };
+    if (!G.slot_done[cur][s]) {
+        const uint32_t* key = G.slot_box[cur] + kBoxWords * s;
+        float box[6], cmn[3], cmx[3];
+        for (int a = 0; a < 3; ++a) {
+            box[a] = fdec(key[a]); box[3 + a] = fdec(key[3 + a]);
+            cmn[a] = fdec(key[6 + a]); cmx[a] = fdec(key[9 + a]);
+        }
+        zero_fix(C, idx, box, key + 12);
+        uint32_t axis, pos, nl;
+        const float cost = warp_sweep(G.bins + (size_t)s * 3 * C.bins * kBinWords, C.bins, cmn, cmx, lane, axis, pos, nl);
+        P = plan_from(C, cost, axis, pos, nl, count, box, box + 3, cmn, cmx);
+        // the element at position nl decides where the front part ends
+        if (P.partition && P.nl < count) P.p = P.nl + (goes_left(C, P, idx[first + P.nl]) ? 0u : 1u);
+        if (lane == 0) {
+            C.ta[X] = make_float4(box[0], box[1], box[2], __uint_as_float(first));
+            C.tb[X] = make_float4(box[3], box[4], box[5], __uint_as_float(count));
+        }
+        if (P.children) {
+            uint32_t L = 0;
+            if (lane == 0) {
+                L = atomicAdd(&C.tcount[0], 2u);
+                const uint32_t d = C.tdepth[X] + 1;
+                for (uint32_t q = 0; q < 2; ++q) {
+                    C.ta[L + q] = make_float4(0, 0, 0, __uint_as_float(q ? first + P.nl : first));
+                    C.tb[L + q] = make_float4(0, 0, 0, __uint_as_float(q ? count - P.nl : P.nl));
+                    C.tleft[L + q] = kNone;
+                    C.tparent[L + q] = X;
+                    C.tdepth[L + q] = d;
+                }
+                C.tleft[X] = L;
+            }
+            L = __shfl_sync(0xffffffffu, L, 0);
+            for (uint32_t q = 0; q < 2; ++q) {
+                const uint32_t c = q ? count - P.nl : P.nl;
+                if (c > kSmall) cs[q] = add_slot(L + q, c, 0u);
+                else if (lane == 0) C.small_list[atomicAdd(&C.tcount[2], 1u)] = L + q;
+            }
+        } else if (P.partition && cur == 0u) {
+            // a rotated leaf lands in idx[1]: the next level moves it back
+            add_slot(X, count, 1u);
+        }
+    }
+    if (lane == 0) {
+        G.plan[s] = P;
+        G.child_slot[2 * s] = cs[0];
+        G.child_slot[2 * s + 1] = cs[1];
     }
 }
 
-__global__ void __launch_bounds__(kChunkThreads) k_child_bounds(Ctx C, Level Lv) {
-    uint32_t slot, first, count, i0, i1;
-    if (!chunk_of(C, Lv, blockIdx.x, slot, first, count, i0, i1)) return;
-    const Plan P = Lv.plan[slot];
-    if (!P.children) return;
-    const uint32_t j0 = Lv.child_slot[2 * slot], j1 = Lv.child_slot[2 * slot + 1];
-    if (j0 == kNone && j1 == kNone) return;
+// A chunk's side bits and its left-goers.
+__device__ __forceinline__ void side_chunk(const Ctx& C, const Large& G, uint32_t cur, const uint32_t* idx, uint32_t b,
+                                           uint32_t* s_w) {
+    const Chunk k = chunk_of(C, G, cur, b);
+    const Plan P = G.plan[k.slot];
+    if (!P.partition) return;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t sum = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < 4; ++r) {
+        const uint32_t w = 4 * warp + r, i = k.i0 + 32 * w + lane;
+        const unsigned m = __ballot_sync(0xffffffffu, i < k.i1 && goes_left(C, P, idx[k.first + i]));
+        if (lane == 0) G.side[32 * (size_t)b + w] = m;
+        sum += __popc(m);
+    }
+    if (lane == 0) s_w[warp] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t all = 0;
+        for (uint32_t w = 0; w < kChunkThreads / 32; ++w) all += s_w[w];
+        G.chunk_l[b] = all;
+    }
+    __syncthreads();
+}
+
+// Ranks (MOVE = false) or destinations (true) of a chunk's positions; moving,
+// the bounds of the large children too.  A slot that is not partitioned and
+// lies in idx[1] is copied to idx[0].
+template <bool MOVE>
+__device__ __forceinline__ void part_chunk(const Ctx& C, const Large& G, uint32_t cur, uint32_t b, uint32_t (*s_box)[kBoxWords]) {
+    const Chunk k = chunk_of(C, G, cur, b);
+    const Plan P = G.plan[k.slot];
+    const uint32_t* from = cur ? C.idx[1] : C.idx[0];
+    uint32_t* to = cur ? C.idx[0] : C.idx[1];
+    if (!P.partition) {
+        if (MOVE && cur)
+            for (uint32_t i = k.i0 + threadIdx.x; i < k.i1; i += blockDim.x) to[k.first + i] = from[k.first + i];
+        return;
+    }
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    // left-goers before the chunk, then before each of its 32 words
+    uint32_t pre = 0;
+    for (uint32_t q = G.slot_chunk[cur][k.slot] + lane; q < b; q += 32) pre += G.chunk_l[q];
+    pre = __reduce_add_sync(0xffffffffu, pre);
+    const uint32_t word = G.side[32 * (size_t)b + lane];
+    uint32_t incl = __popc(word);
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += o;
+    }
+    const uint32_t before = pre + incl - __popc(word);
+    uint32_t j0 = kNone, j1 = kNone;
+    if (MOVE) { j0 = G.child_slot[2 * k.slot]; j1 = G.child_slot[2 * k.slot + 1]; }
+    const bool bounds = j0 != kNone || j1 != kNone;
+    if (MOVE && bounds) {
+        if (threadIdx.x < 2 * kBoxWords) s_box[threadIdx.x / kBoxWords][threadIdx.x % kBoxWords] = key_init(threadIdx.x % kBoxWords);
+        __syncthreads();
+    }
     float v0[12], v1[12];
     uint32_t z0[6], z1[6];
     box_init(v0);
     box_init(v1);
     zero_init(z0);
     zero_init(z1);
-    for (uint32_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const uint32_t t = C.idx[first + i];
-        if (i < P.nl) {
-            if (j0 != kNone) { box_add(v0, C, t); zero_add(z0, C, t, first + i); }
+#pragma unroll
+    for (uint32_t r = 0; r < 4; ++r) {
+        const uint32_t w = 4 * warp + r, i = k.i0 + 32 * w + lane;
+        const unsigned m = __shfl_sync(0xffffffffu, word, w);
+        const uint32_t lpre = __shfl_sync(0xffffffffu, before, w) + __popc(m & ((1u << lane) - 1u));
+        if (i >= k.i1) continue;
+        const bool left = (m >> lane) & 1u;
+        if (!MOVE) {
+            partition_rank(C, P, k.first, i, left, lpre);
+            continue;
+        }
+        const uint32_t t = from[k.first + i], dst = partition_dst(C, P, k.first, k.count, i, left, lpre);
+        to[k.first + dst] = t;
+        if (dst < P.nl) {
+            if (j0 != kNone) { box_add(v0, C, t); zero_add(z0, C, t, k.first + dst); }
         } else if (j1 != kNone) {
             box_add(v1, C, t);
-            zero_add(z1, C, t, first + i);
+            zero_add(z1, C, t, k.first + dst);
         }
     }
-    box_warp_reduce(v0);
-    box_warp_reduce(v1);
-    zero_warp_reduce(z0);
-    zero_warp_reduce(z1);
-    if ((threadIdx.x & 31) == 0) {
-        if (j0 != kNone && i0 < P.nl) box_atomic(Lv.next_box + kBoxWords * j0, v0, z0);
-        if (j1 != kNone && i1 > P.nl) box_atomic(Lv.next_box + kBoxWords * j1, v1, z1);
+    if (MOVE && bounds) {
+        __syncwarp();
+        if (j0 != kNone) box_warp_atomic(s_box[0], v0, z0, lane);
+        if (j1 != kNone) box_warp_atomic(s_box[1], v1, z1, lane);
+        __syncthreads();
+        if (threadIdx.x < 2 * kBoxWords) {
+            const uint32_t side = threadIdx.x / kBoxWords, q = threadIdx.x % kBoxWords, j = side ? j1 : j0;
+            if (j != kNone && s_box[side][q] != key_init(q)) box_merge(G.slot_box[cur ^ 1u] + kBoxWords * j, s_box[side][q], q);
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kChunkThreads) k_large(Ctx C, Large G) {
+    __shared__ uint32_t s_bins[3 * kMaxBins * kBinWords];
+    __shared__ uint32_t s_w[kChunkThreads / 32];
+    __shared__ uint32_t s_box[2][kBoxWords];
+    const uint32_t lane = threadIdx.x & 31u, words = 3 * C.bins * kBinWords;
+    uint32_t cur = 0, round = 0;
+    for (;;) {
+        const uint32_t nslots = G.cnt[cur], nchunks = G.cnt[2 + cur], nxt = cur ^ 1u;
+        if (nslots == 0u) return;
+        const uint32_t* idx = cur ? C.idx[1] : C.idx[0];
+        for (uint32_t b = blockIdx.x; b < nchunks; b += gridDim.x) bin_chunk(C, G, cur, idx, b, s_bins);
+        if (blockIdx.x == 0 && threadIdx.x == 0) { G.cnt[nxt] = 0u; G.cnt[2 + nxt] = 0u; }
+        if (!grid_barrier(&G.cnt[4], &C.tcount[3], round)) return;
+        for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslots; s += (gridDim.x * blockDim.x) >> 5)
+            plan_slot(C, G, cur, idx, s, lane);
+        if (!grid_barrier(&G.cnt[4], &C.tcount[3], round)) return;
+        const uint32_t nnext = G.cnt[nxt];
+        for (uint32_t b = blockIdx.x; b < nchunks; b += gridDim.x) side_chunk(C, G, cur, idx, b, s_w);
+        for (uint32_t s = blockIdx.x; s < nnext; s += gridDim.x)
+            bins_reset(G.bins + (size_t)s * words, words, threadIdx.x, blockDim.x);
+        if (!grid_barrier(&G.cnt[4], &C.tcount[3], round)) return;
+        for (uint32_t b = blockIdx.x; b < nchunks; b += gridDim.x) part_chunk<false>(C, G, cur, b, s_box);
+        if (!grid_barrier(&G.cnt[4], &C.tcount[3], round)) return;
+        for (uint32_t b = blockIdx.x; b < nchunks; b += gridDim.x) part_chunk<true>(C, G, cur, b, s_box);
+        if (!grid_barrier(&G.cnt[4], &C.tcount[3], round)) return;
+        cur = nxt;
     }
 }
 
@@ -694,13 +754,6 @@ static_assert(kSmall <= 128, "task words hold 8-bit counts and first positions")
 
 __host__ __device__ constexpr size_t small_smem_bytes(uint32_t bins) {
     return (9ull + 1ull + 2ull) * 4ull * kSmall + 4ull * 2ull * kSmall + 4ull * 3ull * bins * kBinWords * kSmallWarps;
-}
-
-// Warp-wide bounds from per-lane folds: v = node min / max, centroid min / max.
-__device__ __forceinline__ void box_warp_redux(float* v) {
-#pragma unroll
-    for (int k = 0; k < 12; ++k)
-        v[k] = fdec((k % 6) < 3 ? __reduce_min_sync(0xffffffffu, fenc(v[k])) : __reduce_max_sync(0xffffffffu, fenc(v[k])));
 }
 
 // The cheapest plane of a node of c <= kDirect triangles (see above): what
@@ -883,7 +936,7 @@ __device__ __forceinline__ uint32_t small_node(const Ctx& C, const SmallSmem& S,
     return P.children ? P.nl : 0u;
 }
 
-__global__ void __launch_bounds__(32 * kSmallWarps) k_small(Ctx C, uint32_t nsmall, uint32_t tcap) {
+__global__ void __launch_bounds__(32 * kSmallWarps) k_small(Ctx C, uint32_t tcap) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ uint32_t s_count[2], s_base, s_splits;
     SmallSmem S;
@@ -898,12 +951,14 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(Ctx C, uint32_t nsma
     S.bins = reinterpret_cast<uint32_t*>(S.G + kSmall);
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     uint32_t* bins = S.bins + warp * 3 * C.bins * kBinWords;
+    const uint32_t nsmall = C.tcount[2];
     for (uint32_t w = blockIdx.x; w < nsmall; w += gridDim.x) {
         const uint32_t R = C.small_list[w];
         const uint32_t gfirst = __float_as_uint(C.ta[R].w), count = __float_as_uint(C.tb[R].w);
         uint32_t dep = C.tdepth[R];
+        const uint32_t* from = (dep & 1u) ? C.idx[1] : C.idx[0];
         for (uint32_t i = t; i < count; i += 32 * kSmallWarps) {
-            const uint32_t id = C.idx[gfirst + i];
+            const uint32_t id = from[gfirst + i];
             const float4 c = C.cen[id], mn = C.tmn[id], mx = C.tmx[id];
             S.d[0 * kSmall + i] = c.x;  S.d[1 * kSmall + i] = c.y;  S.d[2 * kSmall + i] = c.z;
             S.d[3 * kSmall + i] = mn.x; S.d[4 * kSmall + i] = mn.y; S.d[5 * kSmall + i] = mn.z;
@@ -935,6 +990,7 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(Ctx C, uint32_t nsma
                 if (nl && lane == 0) {
                     const uint32_t kl = 2u * atomicAdd(&s_splits, 1u);
                     C.tleft[X] = L0 + kl;
+                    C.tparent[L0 + kl] = C.tparent[L0 + kl + 1u] = X;
                     const uint32_t at = atomicAdd(&s_count[cur ^ 1], 2u);
                     S.task[cur ^ 1][at] = f | (nl << 8) | ((kl + 1u) << 16);
                     S.task[cur ^ 1][at + 1] = (f + nl) | ((c - nl) << 8) | ((kl + 2u) << 16);
@@ -948,52 +1004,70 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(Ctx C, uint32_t nsma
             cur ^= 1u;
             if (nodes) ++dep;
         }
-        for (uint32_t i = t; i < count; i += 32 * kSmallWarps) C.idx[gfirst + i] = S.oidx[S.perm[i]];
-        if (t == 0) atomicMax(&C.tcount[1], dep);
+        for (uint32_t i = t; i < count; i += 32 * kSmallWarps) C.idx[0][gfirst + i] = S.oidx[S.perm[i]];
         __syncthreads();
     }
 }
 
 // ---------------------------------------------------------------- renumbering and output
-__global__ void k_internal_count(Ctx C, uint32_t T, uint32_t depth, uint32_t* ic) {
-    const uint32_t stride = gridDim.x * blockDim.x;
+// Two launches instead of two per depth that each read every node (139 + 4 us at
+// 20,480 triangles, 264 + 15 at 499,280).
+//
+// Internal nodes of every subtree, from the leaves up: the second child to
+// arrive at a node sums both and goes on.  On the way each child's word for the
+// way down is set: {parent, what the child's pre-order rank among the internal
+// nodes is above its parent's}.
+__global__ void k_count(Ctx C, uint32_t* arrived, uint32_t* ic, uint2* up) {
+    const uint32_t stride = gridDim.x * blockDim.x, T = C.tcount[0];
     for (uint32_t X = blockIdx.x * blockDim.x + threadIdx.x; X < T; X += stride) {
-        if (C.tdepth[X] != depth) continue;
-        const uint32_t L = C.tleft[X];
-        ic[X] = L == kNone ? 0u : 1u + ic[L] + ic[L + 1];
+        if (C.tdepth[X] == kNone || C.tleft[X] != kNone) continue;   // unused id, or not a leaf
+        uint32_t cur = X, mine = 0;
+        for (;;) {
+            ic[cur] = mine;
+            if (cur == 0u) {
+                C.tcount[1] = mine;
+                break;
+            }
+            const uint32_t p = C.tparent[cur];
+            __threadfence();
+            if (atomicAdd(&arrived[p], 1u) == 0u) break;
+            __threadfence();
+            const uint32_t L = C.tleft[p];
+            const uint32_t a = __ldcg(&ic[L]), b = __ldcg(&ic[L + 1]);
+            up[L] = make_uint2(p, 1u);
+            up[L + 1] = make_uint2(p, 1u + a);
+            mine = 1u + a + b;
+            cur = p;
+        }
     }
 }
 
-__global__ void k_rank(Ctx C, uint32_t T, uint32_t depth, const uint32_t* ic, uint32_t* rank, uint32_t* fidx) {
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t X = blockIdx.x * blockDim.x + threadIdx.x; X < T; X += stride) {
-        if (C.tdepth[X] != depth) continue;
-        const uint32_t L = C.tleft[X];
-        if (L == kNone) continue;
-        const uint32_t r = rank[X];
-        fidx[L] = 2 + 2 * r;
-        fidx[L + 1] = 3 + 2 * r;
-        rank[L] = r + 1;
-        rank[L + 1] = r + 1 + ic[L];
-    }
-}
-
-__global__ void k_emit(Ctx C, uint32_t T, const uint32_t* rank, const uint32_t* fidx, float4* out) {
-    const uint32_t stride = gridDim.x * blockDim.x;
+// The nodes at their places: a node's rank is the sum of the words up to the
+// root; left children have odd ids (pairs are handed out from id 1).
+__global__ void k_emit(Ctx C, const uint2* up, float4* out) {
+    const uint32_t stride = gridDim.x * blockDim.x, T = C.tcount[0];
     for (uint32_t X = blockIdx.x * blockDim.x + threadIdx.x; X < T; X += stride) {
         if (C.tdepth[X] == kNone) continue;   // id reserved by a small subtree but not used
         const float4 a = C.ta[X], b = C.tb[X];
         const bool internal = C.tleft[X] != kNone;
-        const uint32_t f = fidx[X];
-        out[2ull * f] = make_float4(a.x, a.y, a.z, internal ? __uint_as_float(2 + 2 * rank[X]) : a.w);
+        uint32_t rank = 0, above = 0;
+        for (uint32_t cur = X; cur != 0u;) {
+            const uint2 u = up[cur];
+            if (cur == X) above = u.y;
+            rank += u.y;
+            cur = u.x;
+        }
+        const uint32_t f = X == 0u ? 0u : 2u + 2u * (rank - above) + ((X & 1u) ? 0u : 1u);
+        out[2ull * f] = make_float4(a.x, a.y, a.z, internal ? __uint_as_float(2 + 2 * rank) : a.w);
         out[2ull * f + 1] = make_float4(b.x, b.y, b.z, internal ? __uint_as_float(0u) : b.w);
+        if (X == 0u) out[2] = out[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // node 1 is unused
     }
 }
 
 __global__ void k_leaf_tris(Ctx C, float4* out) {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < C.n; i += stride) {
-        const uint32_t t = C.idx[i];
+        const uint32_t t = C.idx[0][i];
         const float* p = C.pos + 9ull * t;
         out[3ull * i] = make_float4(p[0], p[1], p[2], __uint_as_float(t));
         out[3ull * i + 1] = make_float4(p[3] - p[0], p[4] - p[1], p[5] - p[2], 0.0f);
@@ -1019,6 +1093,10 @@ struct DeviceBlock {
     ~DeviceBlock() { dfree(p); }
 };
 
+// k_large's grid: a block per 128 triangles up to 2 per SM (a block per 256 or
+// 512: 356 -> 364 / 385 us at 1,280 triangles; 1 per SM: 2,045 -> 2,199 us at
+// 200,000, 4: the same).
+constexpr uint32_t kLargeBlocksPerSm = 2, kLargePerBlock = 128;
 unsigned blocks_for(uint64_t n, unsigned threads, unsigned cap = 152u * 16u) {
     uint64_t b = (n + threads - 1) / threads;
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(b, cap));
@@ -1053,18 +1131,20 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
     const uint64_t max_nodes = 2ull * n;   // 2 + 2 * (internal nodes <= n - 1)
 
     Arena A;
-    const size_t o_pos = A.part<float>(9ull * n), o_cen = A.part<float4>(n), o_tmn = A.part<float4>(n),
-                 o_tmx = A.part<float4>(n), o_idx = A.part<uint32_t>(n), o_idx_tmp = A.part<uint32_t>(n),
-                 o_F = A.part<uint32_t>(n), o_G = A.part<uint32_t>(n), o_ta = A.part<float4>(tcap),
-                 o_tb = A.part<float4>(tcap), o_tleft = A.part<uint32_t>(tcap), o_tdepth = A.part<uint32_t>(tcap),
-                 o_tcount = A.part<uint32_t>(4), o_small = A.part<uint32_t>(n);
-    const size_t o_st0 = A.part<uint32_t>(maxslots), o_st1 = A.part<uint32_t>(maxslots),
-                 o_sb0 = A.part<uint32_t>(kBoxWords * maxslots), o_sb1 = A.part<uint32_t>(kBoxWords * maxslots),
-                 o_bins = A.part<uint32_t>((size_t)maxslots * 3 * B * kBinWords),
-                 o_choff = A.part<uint32_t>(maxslots + 1), o_chl = A.part<uint32_t>(maxchunks),
+    const size_t o_pos = A.part<float>(9ull * n), o_cen = A.part<float4>(3ull * n), o_idx = A.part<uint32_t>(n),
+                 o_idx_tmp = A.part<uint32_t>(n), o_FG = A.part<uint32_t>(std::max<uint64_t>(2ull * n, tcap)),
+                 o_ta = A.part<float4>(tcap), o_tb = A.part<float4>(tcap), o_tleft = A.part<uint32_t>(tcap),
+                 o_tparent = A.part<uint32_t>(tcap), o_tdepth = A.part<uint32_t>(tcap),
+                 o_tcount = A.part<uint32_t>(4), o_small = A.part<uint32_t>(n), o_ic = A.part<uint32_t>(tcap);
+    size_t o_par[2][5];
+    for (auto& q : o_par) {
+        q[0] = A.part<uint32_t>(maxslots); q[1] = A.part<uint32_t>((size_t)kBoxWords * maxslots);
+        q[2] = A.part<uint32_t>(maxslots); q[3] = A.part<uint32_t>(maxslots); q[4] = A.part<uint32_t>(maxchunks);
+    }
+    const size_t o_bins = A.part<uint32_t>((size_t)maxslots * 3 * B * kBinWords),
+                 o_chl = A.part<uint32_t>(maxchunks), o_side = A.part<uint32_t>(32ull * maxchunks),
                  o_plan = A.part<Plan>(maxslots), o_child = A.part<uint32_t>(2ull * maxslots),
-                 o_next = A.part<uint32_t>(1), o_ic = A.part<uint32_t>(tcap), o_rank = A.part<uint32_t>(tcap),
-                 o_fidx = A.part<uint32_t>(tcap);
+                 o_cnt = A.part<uint32_t>(5);
     const size_t o_nodes = out->keep_device ? 0 : A.part<float4>(2 * max_nodes);
     DeviceBlock scratch;
     {
@@ -1093,117 +1173,60 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
     C.n = n; C.bins = B; C.single = o.subdivide_single_prim ? 1u : 0u; C.max_leaf = o.max_leaf_prims;
     float* d_pos = static_cast<float*>(at(o_pos));
     C.pos = d_pos;
-    C.cen = static_cast<float4*>(at(o_cen)); C.tmn = static_cast<float4*>(at(o_tmn));
-    C.tmx = static_cast<float4*>(at(o_tmx));
-    C.idx = static_cast<uint32_t*>(at(o_idx)); C.idx_tmp = static_cast<uint32_t*>(at(o_idx_tmp));
-    C.F = static_cast<uint32_t*>(at(o_F)); C.G = static_cast<uint32_t*>(at(o_G));
+    C.cen = static_cast<float4*>(at(o_cen)); C.tmn = C.cen + n; C.tmx = C.tmn + n;
+    C.idx[0] = static_cast<uint32_t*>(at(o_idx)); C.idx[1] = static_cast<uint32_t*>(at(o_idx_tmp));
+    C.F = static_cast<uint32_t*>(at(o_FG)); C.G = C.F + n;
     C.ta = static_cast<float4*>(at(o_ta)); C.tb = static_cast<float4*>(at(o_tb));
-    C.tleft = static_cast<uint32_t*>(at(o_tleft)); C.tdepth = static_cast<uint32_t*>(at(o_tdepth));
+    C.tleft = static_cast<uint32_t*>(at(o_tleft)); C.tparent = static_cast<uint32_t*>(at(o_tparent));
+    C.tdepth = static_cast<uint32_t*>(at(o_tdepth));
     C.tcount = static_cast<uint32_t*>(at(o_tcount));
     C.small_list = static_cast<uint32_t*>(at(o_small));
-    uint32_t* slot_tmp[2] = {static_cast<uint32_t*>(at(o_st0)), static_cast<uint32_t*>(at(o_st1))};
-    uint32_t* slot_box[2] = {static_cast<uint32_t*>(at(o_sb0)), static_cast<uint32_t*>(at(o_sb1))};
-    uint32_t* bins = static_cast<uint32_t*>(at(o_bins));
-    uint32_t* chunk_off = static_cast<uint32_t*>(at(o_choff));
-    uint32_t* chunk_l = static_cast<uint32_t*>(at(o_chl));
-    Plan* plan = static_cast<Plan*>(at(o_plan));
-    uint32_t* child_slot = static_cast<uint32_t*>(at(o_child));
-    uint32_t* next_count = static_cast<uint32_t*>(at(o_next));
+    Large G{};
+    for (int q = 0; q < 2; ++q) {
+        G.slot_tmp[q] = static_cast<uint32_t*>(at(o_par[q][0]));
+        G.slot_box[q] = static_cast<uint32_t*>(at(o_par[q][1]));
+        G.slot_done[q] = static_cast<uint32_t*>(at(o_par[q][2]));
+        G.slot_chunk[q] = static_cast<uint32_t*>(at(o_par[q][3]));
+        G.chunk_slot[q] = static_cast<uint32_t*>(at(o_par[q][4]));
+    }
+    G.bins = static_cast<uint32_t*>(at(o_bins)); G.chunk_l = static_cast<uint32_t*>(at(o_chl));
+    G.side = static_cast<uint32_t*>(at(o_side)); G.plan = static_cast<Plan*>(at(o_plan));
+    G.child_slot = static_cast<uint32_t*>(at(o_child)); G.cnt = static_cast<uint32_t*>(at(o_cnt));
+    // free once the tree stands: the partition's ranks take the arrivals, the
+    // triangles' boxes the words up the tree (2 tcap words in 12 n)
+    uint32_t* arrived = C.F;
+    uint2* up = reinterpret_cast<uint2*>(C.cen);
     uint32_t* ic = static_cast<uint32_t*>(at(o_ic));
-    uint32_t* rank = static_cast<uint32_t*>(at(o_rank));
-    uint32_t* fidx = static_cast<uint32_t*>(at(o_fidx));
 
     BVH_CUDA(cudaMemcpyAsync(d_pos, hpos.get(), 36ull * n, cudaMemcpyHostToDevice, st));
-    k_prep<<<blocks_for(n, 256), 256, 0, st>>>(C);
-    // root = temporary node 0
-    {
-        const float4 a = make_float4(0, 0, 0, 0);
-        float4 b = make_float4(0, 0, 0, 0);
-        uint32_t nn = n;
-        std::memcpy(&b.w, &nn, 4);
-        const uint32_t init[4] = {1u, 0u, 0u, 0u}, none = kNone, zero = 0u;
-        BVH_CUDA(cudaMemcpyAsync(C.ta, &a, 16, cudaMemcpyHostToDevice, st));
-        BVH_CUDA(cudaMemcpyAsync(C.tb, &b, 16, cudaMemcpyHostToDevice, st));
-        BVH_CUDA(cudaMemcpyAsync(C.tleft, &none, 4, cudaMemcpyHostToDevice, st));
-        BVH_CUDA(cudaMemcpyAsync(C.tdepth, &zero, 4, cudaMemcpyHostToDevice, st));
-        BVH_CUDA(cudaMemcpyAsync(C.tcount, init, 16, cudaMemcpyHostToDevice, st));
-        BVH_CUDA(cudaStreamSynchronize(st));   // the host copies above read stack variables
-    }
-    uint32_t nslots = 0;
+    // ids that a small subtree reserves but does not use keep depth kNone
+    BVH_CUDA(cudaMemsetAsync(C.tdepth, 0xFF, 4ull * tcap, st));
+    k_init<<<1, 256, 0, st>>>(C, G);
+    k_prep<<<blocks_for(n, 256, 152u * 4u), 256, 0, st>>>(C, n > kSmall ? G.slot_box[0] : nullptr);
     if (n > kSmall) {
-        const uint32_t zero = 0u;
-        BVH_CUDA(cudaMemcpyAsync(slot_tmp[0], &zero, 4, cudaMemcpyHostToDevice, st));
-        k_keys_init<<<1, 32, 0, st>>>(slot_box[0], kBoxWords);
-        k_root_bounds<<<blocks_for(n, 256), 256, 0, st>>>(C, slot_box[0]);
-        BVH_CUDA(cudaStreamSynchronize(st));
-        nslots = 1;
-    } else {
-        const uint32_t zero = 0u, one = 1u;
-        BVH_CUDA(cudaMemcpyAsync(C.small_list, &zero, 4, cudaMemcpyHostToDevice, st));
-        BVH_CUDA(cudaMemcpyAsync(C.tcount + 2, &one, 4, cudaMemcpyHostToDevice, st));
-        BVH_CUDA(cudaStreamSynchronize(st));
+        // a cooperative launch: its blocks wait for one another
+        int per_sm = 0;
+        BVH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_large, kChunkThreads, 0));
+        const unsigned most = (unsigned)sm_count() * (unsigned)std::max(1, std::min(per_sm, (int)kLargeBlocksPerSm));
+        const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(most, n / kLargePerBlock));
+        void* args[] = {&C, &G};
+        BVH_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_large), dim3(grid), dim3(kChunkThreads), args, 0, st));
     }
-    int cur = 0;
-    while (nslots > 0) {
-        Level Lv;
-        Lv.nslots = nslots;
-        Lv.slot_tmp = slot_tmp[cur];
-        Lv.slot_box = slot_box[cur];
-        Lv.bins = bins;
-        Lv.chunk_off = chunk_off;
-        Lv.chunk_l = chunk_l;
-        Lv.plan = plan;
-        Lv.child_slot = child_slot;
-        Lv.next_tmp = slot_tmp[cur ^ 1];
-        Lv.next_box = slot_box[cur ^ 1];
-        Lv.next_count = next_count;
-        // chunks in this level: sum of ceil(count / kChunk) <= n / kChunk + nslots
-        const unsigned grid = (unsigned)std::min<uint64_t>(maxchunks, (uint64_t)n / kChunk + nslots + 1);
-        const unsigned sgrid = (nslots + 127) / 128;
-        BVH_CUDA(cudaMemsetAsync(next_count, 0, 4, st));
-        k_chunk_scan<<<1, 1024, 0, st>>>(C, Lv);
-        k_bins_reset<<<blocks_for((uint64_t)nslots * 3 * B * kBinWords, 256), 256, 0, st>>>(C, Lv);
-        k_bin_chunks<<<grid, kChunkThreads, 0, st>>>(C, Lv);
-        k_plan<<<(nslots + 3) / 4, 128, 0, st>>>(C, Lv);
-        k_part_count<<<grid, kChunkThreads, 0, st>>>(C, Lv);
-        k_part_slot_scan<<<sgrid, 128, 0, st>>>(C, Lv);
-        k_part_pass<false><<<grid, kChunkThreads, 0, st>>>(C, Lv);
-        k_part_pass<true><<<grid, kChunkThreads, 0, st>>>(C, Lv);
-        k_part_copy<<<grid, kChunkThreads, 0, st>>>(C, Lv);
-        k_children<<<sgrid, 128, 0, st>>>(C, Lv);
-        k_child_bounds<<<grid, kChunkThreads, 0, st>>>(C, Lv);
-        BVH_CUDA(cudaGetLastError());
-        BVH_CUDA(cudaMemcpyAsync(&nslots, next_count, 4, cudaMemcpyDeviceToHost, st));
-        BVH_CUDA(cudaStreamSynchronize(st));
-        cur ^= 1;
-    }
+    const size_t smem = small_smem_bytes(B);
+    BVH_CUDA(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_small<<<blocks_for(n, 48, 1u << 16), 32 * kSmallWarps, smem, st>>>(C, (uint32_t)tcap);
+    BVH_CUDA(cudaMemsetAsync(arrived, 0, 4ull * tcap, st));
+    k_count<<<blocks_for(tcap, 256), 256, 0, st>>>(C, arrived, ic, up);
+    BVH_CUDA(cudaGetLastError());
     uint32_t counts[4];
-    BVH_CUDA(cudaMemcpyAsync(counts, C.tcount, 12, cudaMemcpyDeviceToHost, st));
-    BVH_CUDA(cudaStreamSynchronize(st));
-    if (counts[2] > 0) {
-        // ids from counts[0] on are reserved per small subtree; unused ones keep depth kNone
-        BVH_CUDA(cudaMemsetAsync(C.tdepth + counts[0], 0xFF, 4ull * (tcap - counts[0]), st));
-        const size_t smem = small_smem_bytes(B);
-        BVH_CUDA(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_small<<<counts[2], 32 * kSmallWarps, smem, st>>>(C, counts[2], (uint32_t)tcap);
-        BVH_CUDA(cudaGetLastError());
-    }
     BVH_CUDA(cudaMemcpyAsync(counts, C.tcount, 16, cudaMemcpyDeviceToHost, st));
     BVH_CUDA(cudaStreamSynchronize(st));
     if (counts[3] != 0) {
-        g_err = "gpu_bvh_build: small-subtree node ids exceeded the reserved range";
-        return WF_ERR_CAPACITY;
+        g_err = (counts[3] & 2u) ? "gpu_bvh_build: a grid barrier gave up"
+                                 : "gpu_bvh_build: small-subtree node ids exceeded the reserved range";
+        return (counts[3] & 2u) ? WF_ERR_TIMEOUT : WF_ERR_CAPACITY;
     }
-    const uint32_t T = counts[0], maxd = counts[1];
-    const unsigned tgrid = blocks_for(T, 256);
-    for (int d = (int)maxd; d >= 0; --d) k_internal_count<<<tgrid, 256, 0, st>>>(C, T, (uint32_t)d, ic);
-    BVH_CUDA(cudaMemsetAsync(rank, 0, 4, st));
-    BVH_CUDA(cudaMemsetAsync(fidx, 0, 4, st));
-    for (uint32_t d = 0; d < maxd; ++d) k_rank<<<tgrid, 256, 0, st>>>(C, T, d, ic, rank, fidx);
-    uint32_t internal = 0;
-    BVH_CUDA(cudaMemcpyAsync(&internal, ic, 4, cudaMemcpyDeviceToHost, st));
-    BVH_CUDA(cudaStreamSynchronize(st));
-    const uint32_t nc = 2 + 2 * internal;
+    const uint32_t nc = 2 + 2 * counts[1];
     float4* d_nodes = nullptr;
     float4* d_tris = nullptr;
     if (out->keep_device) {
@@ -1223,8 +1246,8 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
             dfree(d_tris);
         }
     };
-    cudaError_t e = cudaMemsetAsync(d_nodes, 0, 32ull * nc, st);
-    k_emit<<<tgrid, 256, 0, st>>>(C, T, rank, fidx, d_nodes);
+    cudaError_t e = cudaSuccess;
+    k_emit<<<blocks_for(counts[0], 256), 256, 0, st>>>(C, up, d_nodes);
     if (d_tris) k_leaf_tris<<<blocks_for(n, 256), 256, 0, st>>>(C, d_tris);
     if (e == cudaSuccess) e = cudaGetLastError();
     // blob: [header | nodes | bvh_triangle_t (original order) | index list], written
@@ -1243,7 +1266,7 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
     out->blob_size = size;
     if (e == cudaSuccess) e = cudaMemcpyAsync(blob + 12, d_nodes, nodes_bytes, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(blob + 12 + nodes_bytes + tri_bytes, C.idx, idx_bytes, cudaMemcpyDeviceToHost, st);
+        e = cudaMemcpyAsync(blob + 12 + nodes_bytes + tri_bytes, C.idx[0], idx_bytes, cudaMemcpyDeviceToHost, st);
     uint8_t* tri_dst = blob + 12 + nodes_bytes;
     host_parallel(tri_bytes, 1u << 22, [&](uint64_t lo, uint64_t hi) {
         std::memcpy(tri_dst + lo, reinterpret_cast<const uint8_t*>(hpos.get()) + lo, hi - lo);

@@ -54,5 +54,6 @@ void host_parallel(uint64_t n, uint64_t grain, F f) {
 // The library's accounted device allocator (wf_api.cu).
 cudaError_t dmalloc(void** p, size_t bytes);
 void dfree(void* p);
+int sm_count();
 
 }  // namespace wf
