@@ -621,13 +621,96 @@ namespace {
 std::mutex g_mem_mutex;
 std::unordered_map<void*, size_t> g_mem_blocks;
 uint64_t g_mem_used = 0, g_mem_limit = 0;   // limit 0: none
+
+// Scratch blocks kept between calls (cudaMalloc + cudaFree of a build's scratch
+// take 75 us for a few MB and 130 us for 130 MB, and cudaFree waits for the
+// whole device).  A kept block is idle: its last user's stream was synchronized
+// before it came back.  At most kKeptBytes are kept; all go back to the driver
+// when an allocation fails, when the memory limit leaves no room for them and
+// when the last context is destroyed.  Idle blocks do not count as used.
+struct Kept {
+    void* p;
+    size_t bytes;
+    int device;
+};
+constexpr uint64_t kKeptBytes = 256ull << 20;
+std::vector<Kept> g_kept;
+uint64_t g_kept_bytes = 0;
+uint32_t g_contexts = 0;
+
+void drop_kept() {   // g_mem_mutex held
+    for (const Kept& k : g_kept) cudaFree(k.p);
+    g_kept.clear();
+    g_kept_bytes = 0;
+}
 }  // namespace
+
+// Contexts alive: the kept blocks go with the last one.
+static void count_context(int by) {
+    std::lock_guard<std::mutex> lock(g_mem_mutex);
+    g_contexts += (uint32_t)by;
+    if (g_contexts == 0) drop_kept();
+}
+
+cudaError_t scratch_take(void** p, size_t bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(g_mem_mutex);
+        size_t best = g_kept.size();
+        for (size_t i = 0; i < g_kept.size(); ++i)
+            if (g_kept[i].device == dev && g_kept[i].bytes >= bytes &&
+                (best == g_kept.size() || g_kept[i].bytes < g_kept[best].bytes))
+                best = i;
+        if (best < g_kept.size() && !(g_mem_limit && g_mem_used + g_kept[best].bytes > g_mem_limit)) {
+            const Kept k = g_kept[best];
+            g_kept.erase(g_kept.begin() + (long)best);
+            g_kept_bytes -= k.bytes;
+            g_mem_blocks[k.p] = k.bytes;
+            g_mem_used += k.bytes;
+            *p = k.p;
+            return cudaSuccess;
+        }
+    }
+    return dmalloc(p, bytes);
+}
+
+void scratch_give(void* p) {
+    if (!p) return;
+    int dev = 0;
+    const bool have = cudaGetDevice(&dev) == cudaSuccess;
+    {
+        std::lock_guard<std::mutex> lock(g_mem_mutex);
+        auto it = g_mem_blocks.find(p);
+        const size_t bytes = it == g_mem_blocks.end() ? 0 : it->second;
+        if (have && bytes && g_contexts && bytes <= kKeptBytes &&
+            !(g_mem_limit && g_mem_used + g_kept_bytes > g_mem_limit)) {
+            // the newest stays; older ones make room
+            while (!g_kept.empty() && g_kept_bytes + bytes > kKeptBytes) {
+                cudaFree(g_kept.front().p);
+                g_kept_bytes -= g_kept.front().bytes;
+                g_kept.erase(g_kept.begin());
+            }
+            g_mem_blocks.erase(it);
+            g_mem_used -= bytes;
+            g_kept.push_back(Kept{p, bytes, dev});
+            g_kept_bytes += bytes;
+            return;
+        }
+    }
+    dfree(p);
+}
 
 cudaError_t dmalloc(void** p, size_t bytes) {
     *p = nullptr;
     std::lock_guard<std::mutex> lock(g_mem_mutex);
+    if (g_mem_limit && g_mem_used + g_kept_bytes + bytes > g_mem_limit) drop_kept();
     if (g_mem_limit && g_mem_used + bytes > g_mem_limit) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && !g_kept.empty()) {
+        cudaGetLastError();
+        drop_kept();
+        e = cudaMalloc(p, bytes);
+    }
     if (e != cudaSuccess) {
         *p = nullptr;
         return e;
@@ -809,6 +892,7 @@ int wf_checked_build(void) { return WF_CHECKED; }
 int wf_set_device_memory_limit(uint64_t bytes) {
     std::lock_guard<std::mutex> lock(g_mem_mutex);
     g_mem_limit = bytes;
+    if (bytes && g_mem_used + g_kept_bytes > bytes) drop_kept();
     return WF_OK;
 }
 
@@ -832,20 +916,24 @@ int wf_create(const wf_init_params* p, wf_ctx** out) {
     }
     if (p->device < 0 || p->device >= ndev) return fail(WF_ERR_INVALID, "wf_create: device ordinal out of range");
     wf_ctx* c = new wf_ctx();
+    count_context(1);
     c->device = p->device;
     c->width = p->render_width;
     c->height = p->render_height;
     if (p->tlas_metric > 3) {
         delete c;
+        count_context(-1);
         return fail(WF_ERR_INVALID, "wf_create: tlas_metric must be 0, 1, 2 or 3");
     }
     c->tlas_metric = p->tlas_metric;
     if (p->blas_layout > 2) {
         delete c;
+        count_context(-1);
         return fail(WF_ERR_INVALID, "wf_create: blas_layout must be 0, 1 or 2");
     }
     if (p->instance_bounds > 1) {
         delete c;
+        count_context(-1);
         return fail(WF_ERR_INVALID, "wf_create: instance_bounds must be 0 or 1");
     }
     c->blas_layout = p->blas_layout;
@@ -921,6 +1009,7 @@ int wf_destroy(wf_ctx* c) {
     if (c->img_copied) cudaEventDestroy(c->img_copied);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
+    count_context(-1);
     return WF_OK;
 }
 

@@ -33,9 +33,11 @@
 // shared-memory bins, side bits and chunked scans for the partition); subtrees
 // of at most kSmall triangles are built by one CTA each, entirely in shared
 // memory; the renumbering climbs from the leaves once and from every node once.
-// Nothing is read back before the tree stands.  The host side makes one scratch allocation,
-// gathers the positions on several threads and writes the blob straight into
-// the caller's buffer when it fits.
+// Nothing is read back before the tree stands.  The scratch is one allocation,
+// kept for the next build when it is small; the triangles go to the device as
+// they are (144 bytes each, over NVLink-C2C) and their positions are picked out
+// there, and the blob's three parts are copied straight into the caller's buffer
+// when it fits.
 #include <algorithm>
 #include <cstring>
 #include <memory>
@@ -355,8 +357,8 @@ __device__ __forceinline__ void bins_reset(uint32_t* sb, uint32_t words, uint32_
 // with the level's node count read back by the host, took about 100 us per
 // level however few triangles it had; us per wf_bvh_build, so / in one launch,
 // with the renumbering below: 80 triangles 296 / 190, 1,280: 672 / 356, 20,480:
-// 1,634 / 851, 100,820: 2,684 / 1,560, 499,280: 7,423 / 6,180 (4.8 ms of it the
-// host's copies).
+// 1,634 / 851, 100,820: 2,684 / 1,560, 499,280: 7,423 / 6,180 (0.98 ms of it
+// k_large, 0.97 k_small, most of the rest the host's).
 //
 // A slot is a node of the level, a chunk kChunk consecutive positions of one
 // slot; a block takes chunks in turn.  Slots and chunks of the next level are
@@ -395,6 +397,15 @@ __global__ void k_init(Ctx C, Large G) {
     if (!large) return;
     for (uint32_t k = t; k < nch; k += blockDim.x) G.chunk_slot[0][k] = 0u;
     bins_reset(G.bins, 3 * C.bins * kBinWords, t, blockDim.x);
+}
+
+// Positions {v0, v1, v2} of m triangle_t (three 48-byte vertices each).
+__global__ void k_gather(const float4* __restrict__ tris, uint32_t m, float* __restrict__ pos) {
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < 3 * m; q += stride) {
+        const float4 p = tris[3ull * q];
+        pos[3ull * q] = p.x; pos[3ull * q + 1] = p.y; pos[3ull * q + 2] = p.z;
+    }
 }
 
 // Centroid and box per triangle, and the root's bounds.
@@ -1088,9 +1099,15 @@ struct Arena {
     }
 };
 
+// A build's scratch: back to the kept blocks once the stream is done with it,
+// else (an error on the way) freed, which waits.
 struct DeviceBlock {
     void* p = nullptr;
-    ~DeviceBlock() { dfree(p); }
+    bool done = false;
+    ~DeviceBlock() {
+        if (done) scratch_give(p);
+        else dfree(p);
+    }
 };
 
 // k_large's grid: a block per 128 triangles up to 2 per SM (a block per 256 or
@@ -1148,7 +1165,7 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
     const size_t o_nodes = out->keep_device ? 0 : A.part<float4>(2 * max_nodes);
     DeviceBlock scratch;
     {
-        const cudaError_t e = dmalloc(&scratch.p, A.bytes);
+        const cudaError_t e = scratch_take(&scratch.p, A.bytes);
         if (e != cudaSuccess) {
             cudaGetLastError();
             g_err = std::string("gpu_bvh_build: cudaMalloc: ") + cudaGetErrorString(e);
@@ -1157,17 +1174,6 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
     }
     uint8_t* base = static_cast<uint8_t*>(scratch.p);
     auto at = [base](size_t off) { return static_cast<void*>(base + off); };
-
-    // triangle positions, gathered on the host threads
-    std::unique_ptr<float[]> hpos(new (std::nothrow) float[9ull * n]);
-    if (!hpos) { g_err = "gpu_bvh_build: host allocation failed"; return WF_ERR_OOM; }
-    host_parallel(n, 1u << 16, [&](uint64_t lo, uint64_t hi) {
-        for (uint64_t i = lo; i < hi; ++i) {
-            std::memcpy(&hpos[9 * i], tris[i].v0.position, 12);
-            std::memcpy(&hpos[9 * i + 3], tris[i].v1.position, 12);
-            std::memcpy(&hpos[9 * i + 6], tris[i].v2.position, 12);
-        }
-    });
 
     Ctx C{};
     C.n = n; C.bins = B; C.single = o.subdivide_single_prim ? 1u : 0u; C.max_leaf = o.max_leaf_prims;
@@ -1198,7 +1204,13 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
     uint2* up = reinterpret_cast<uint2*>(C.cen);
     uint32_t* ic = static_cast<uint32_t*>(at(o_ic));
 
-    BVH_CUDA(cudaMemcpyAsync(d_pos, hpos.get(), 36ull * n, cudaMemcpyHostToDevice, st));
+    // the triangles in turns through the words of the node table, not used yet
+    const uint64_t turn = std::min<uint64_t>(n, 32ull * tcap / sizeof(triangle_t));
+    for (uint64_t t0 = 0; t0 < n; t0 += turn) {
+        const uint32_t m = (uint32_t)std::min<uint64_t>(turn, n - t0);
+        BVH_CUDA(cudaMemcpyAsync(C.ta, tris + t0, m * sizeof(triangle_t), cudaMemcpyHostToDevice, st));
+        k_gather<<<blocks_for(m, 256), 256, 0, st>>>(C.ta, m, d_pos + 9 * t0);
+    }
     // ids that a small subtree reserves but does not use keep depth kNone
     BVH_CUDA(cudaMemsetAsync(C.tdepth, 0xFF, 4ull * tcap, st));
     k_init<<<1, 256, 0, st>>>(C, G);
@@ -1266,17 +1278,16 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
     out->blob_size = size;
     if (e == cudaSuccess) e = cudaMemcpyAsync(blob + 12, d_nodes, nodes_bytes, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
+        e = cudaMemcpyAsync(blob + 12 + nodes_bytes, d_pos, tri_bytes, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
         e = cudaMemcpyAsync(blob + 12 + nodes_bytes + tri_bytes, C.idx[0], idx_bytes, cudaMemcpyDeviceToHost, st);
-    uint8_t* tri_dst = blob + 12 + nodes_bytes;
-    host_parallel(tri_bytes, 1u << 22, [&](uint64_t lo, uint64_t hi) {
-        std::memcpy(tri_dst + lo, reinterpret_cast<const uint8_t*>(hpos.get()) + lo, hi - lo);
-    });
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         drop();
         g_err = std::string("gpu_bvh_build: ") + cudaGetErrorString(e);
         return WF_ERR_CUDA;
     }
+    scratch.done = true;
     bvh_header_t h;
     h.nodes_offset = 12;
     h.triangles_offset = (uint32_t)(12 + nodes_bytes);

@@ -54,6 +54,10 @@ void host_parallel(uint64_t n, uint64_t grain, F f) {
 // The library's accounted device allocator (wf_api.cu).
 cudaError_t dmalloc(void** p, size_t bytes);
 void dfree(void* p);
+// Scratch of a call that has finished with it when it returns (its stream
+// synchronized): a kept block of the current device that fits, else a new one.
+cudaError_t scratch_take(void** p, size_t bytes);
+void scratch_give(void* p);
 int sm_count();
 
 }  // namespace wf
