@@ -336,8 +336,10 @@ int wf_scene_set_emission(wf_ctx* ctx, uint32_t instance, float strength);
  * produces with accumulate = 0: dloss_dimage = d(loss)/d(average radiance),
  * 3 floats per pixel (row-major); writes d(loss)/d(albedo) (3 floats per scene
  * triangle) and d(loss)/d(emissive_strength) (1 per instance).  Each wave is
- * traced once forward (path radiance L) and replayed from the same per-path
- * seeds (w = dloss_dimage / spp, atomics, memory O(paths), no tape): a Lambert
+ * traced once forward (path radiance L, and per path and depth of the wave the
+ * 20 bytes of what its ray hit, at most 4 GiB: the wave is as long as that
+ * allows) and replayed from the same per-path seeds and those hits (w =
+ * dloss_dimage / spp, atomics, no gradient tape): a Lambert
  * vertex adds w*(L - L_before)/albedo, L_before being what the path gathered
  * before it (everything after it, its next-event shadow ray included, is
  * linear in its albedo); each emitted contribution c (an emission hit, or an

@@ -145,10 +145,10 @@ struct wf_ctx {
     bool albedo_set = false;
     DevBuf<float4> tri_albedo;              // per scene triangle (wf_scene_set_albedo)
     DevBuf<uint32_t> inst_tri_offset;
-    DevBuf<float4> L_final, dimage, g_albedo;   // adjoint buffers
-    DevBuf<float> g_emission;
-    DevBuf<float> g_em_rep;                 // adjoint: shadow rays' emitter gradients, 32 replicas
-    DevBuf<float4> L_comp, L_final_lo;      // adjoint: rounding errors of the path radiance sums
+    DevBuf<float4> dimage, g_albedo;        // adjoint buffers
+    DevBuf<float> g_em_rep;                 // adjoint: emitter gradients, 32 replicas
+    DevBuf<float4> L_comp;                  // adjoint: rounding errors of the path radiance sums
+    DevBuf<uint8_t> tape;                   // adjoint: the forward pass's hits and visibilities
 
     // wavefront buffers
     bool buffers_ready = false;
@@ -990,8 +990,8 @@ int wf_destroy(wf_ctx* c) {
     release_buffers(c);
     c->tnodes.release(); c->tinst.release(); c->sinst.release(); c->blas.release(); c->stri.release();
     c->lights.release(); c->aabbs.release(); c->tlas_scratch.release();
-    c->tri_albedo.release(); c->inst_tri_offset.release(); c->L_final.release(); c->dimage.release();
-    c->g_albedo.release(); c->g_emission.release();
+    c->tri_albedo.release(); c->inst_tri_offset.release(); c->dimage.release();
+    c->g_albedo.release(); c->g_em_rep.release(); c->L_comp.release(); c->tape.release();
     c->image.release(); c->image_ldr.release(); c->trace_io.release(); c->sort_scratch.release();
     dev_free(c->status); dev_free(c->counters); dev_free(c->totals); dev_free(c->trace_fetch);
     for (EventPair& p : c->events) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
@@ -1508,7 +1508,7 @@ Pass make_pass(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
 }
 
 // One wave through generate -> (extend -> shade -> connect) x depth [-> resolve].
-int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, const AdjointRefs& A, bool resolve) {
+int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, bool resolve) {
     WaveParams& W = P.W;
     RenderBuffers& B = P.B;
     W.s0 = sample_base + wv.s0;
@@ -1537,7 +1537,7 @@ int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, const Adj
     // whose queue, projected from the last wave's sizes, is below tail_paths
     uint32_t tail = kMaxDepth;
     // whether the extension launch of depth d also traces the shadow rays of d - 1
-    auto fused_at = [&](uint32_t d) { return P.fused || (P.fuse_from != 0 && d >= P.fuse_from && !A.g_em_rep); };
+    auto fused_at = [&](uint32_t d) { return P.fused || (P.fuse_from != 0 && d >= P.fuse_from); };
     if (c->counts_pending) {
         const cudaError_t q = cudaEventQuery(c->ev_counts);
         if (q == cudaSuccess) {
@@ -1550,7 +1550,7 @@ int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, const Adj
             WF_CUDA(q);
         }
     }
-    const bool tail_ok = !P.cnt && A.g_albedo == nullptr && P.tail_paths != 0u && c->counts_known;
+    const bool tail_ok = !P.cnt && P.tail_paths != 0u && c->counts_known;
     if (tail_ok) {
         const uint64_t limit = P.tail_paths;
         for (uint32_t d = 1; d <= W.max_bounces; ++d) {
@@ -1559,7 +1559,7 @@ int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, const Adj
         }
     }
     // A short wave without shadow rays runs whole in one launch.
-    const bool whole = W.npaths <= kWholePaths && !P.nee && !P.prof && !P.cnt && P.S.qbvh == 0u && !A.g_albedo &&
+    const bool whole = W.npaths <= kWholePaths && !P.nee && !P.prof && !P.cnt && P.S.qbvh == 0u &&
                        !B.ps_Lc && W.view_mode == 0u && P.tail_paths == 0u;
     if (whole) {
         WF_CUDA(launch_finish(P.S, P.SH, B, W, 0, c->totals, c->stream));
@@ -1602,7 +1602,7 @@ int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, const Adj
         }
         {
             StageTimer t(c, P.prof, ST_SHADE);
-            WF_CUDA(launch_shade(P.SH, B, W, d, W.npaths, A, c->stream));
+            WF_CUDA(launch_shade(P.SH, B, W, d, W.npaths, c->stream));
         }
         c->launches += 2;
         c->launches_extend++;
@@ -1619,13 +1619,7 @@ int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, const Adj
             }
             {
                 StageTimer t(c, P.prof, ST_CONNECT, cs, (int)d);
-                if (A.g_em_rep) {
-                    const AdjConnect adj{A.dimage, P.SH.sinst, A.g_em_rep, A.instances, W.pix0, W.nsamples,
-                                         A.inv_spp};
-                    WF_CUDA(launch_connect(P.S, B, d, W.npaths, false, c->totals + 1, cs, &adj));
-                } else {
-                    WF_CUDA(launch_connect(P.S, B, d, W.npaths, P.cnt, c->totals + 1, cs));
-                }
+                WF_CUDA(launch_connect(P.S, B, d, W.npaths, P.cnt, c->totals + 1, cs));
             }
             if (!P.serial) {
                 WF_CUDA(cudaEventRecord(c->ev_conn[d], c->side));
@@ -1673,9 +1667,8 @@ int wf_render(wf_ctx* c, const render_settings_t* s, const wf_render_options* o,
     }
     const uint32_t wave = o->wave_paths ? std::min(o->wave_paths, c->capacity) : c->capacity;
     Pass P = make_pass(c, s, o, frame_seed);
-    const AdjointRefs none{};
     for (const Wave& wv : plan_waves(o->spp, npix, wave))
-        if ((rc = run_wave(c, P, wv, c->accum_samples, none, true))) return rc;
+        if ((rc = run_wave(c, P, wv, c->accum_samples, true))) return rc;
     c->accum_samples += o->spp;
     c->last_view_mode = s->render_view_mode;
     c->last_frame_seed = frame_seed;
@@ -1703,55 +1696,71 @@ int wf_adjoint(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
     // gradient replicas spread the atomics of heavily hit triangles; at most 256 MiB
     uint32_t replicas = 32;
     while (replicas > 1 && (uint64_t)replicas * ntri * sizeof(float4) > (256ull << 20)) replicas >>= 1;
-    if ((rc = c->L_final.reserve(c->capacity)) || (rc = c->dimage.reserve(npix)) ||
-        (rc = c->g_albedo.reserve((uint64_t)replicas * ntri)) || (rc = c->g_emission.reserve(ninst)) ||
-        (rc = c->g_em_rep.reserve(32ull * std::max<uint64_t>(ninst, 1))) ||
-        (rc = c->L_comp.reserve(c->capacity)) || (rc = c->L_final_lo.reserve(c->capacity)))
+    if ((rc = c->dimage.reserve(npix)) || (rc = c->g_albedo.reserve((uint64_t)replicas * ntri)) ||
+        (rc = c->g_em_rep.reserve(32ull * std::max<uint64_t>(ninst, 1))) || (rc = c->L_comp.reserve(c->capacity)))
         return rc;
+    // The tape: per path and depth the forward pass's hit (20 bytes) and whether
+    // its shadow ray was unoccluded, so the replay traces no rays.  The wave is
+    // as long as 4 GiB of tape allow; where that much cannot be had, 32 bytes
+    // per path of the context's capacity are enough for shorter waves (results
+    // do not depend on the split).
+    const uint64_t depths = (uint64_t)s->max_bounces + 1, entry = 20 + (o->nee ? 1 : 0);
+    uint32_t wave = o->wave_paths ? std::min(o->wave_paths, c->capacity) : c->capacity;
+    auto tape_paths = [&](uint64_t bytes) {
+        return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(wave, bytes / (depths * entry)));
+    };
+    auto tape_bytes = [&](uint32_t paths) { return depths * entry * paths; };
+    uint32_t tape_wave = tape_paths(4ull << 30);
+    if ((rc = c->tape.reserve(tape_bytes(tape_wave))) == WF_ERR_OOM) {
+        tape_wave = tape_paths(32ull * c->capacity);
+        rc = c->tape.reserve(tape_bytes(tape_wave));
+    }
+    if (rc) return rc;
+    wave = tape_wave;
     std::vector<float4> dimg(npix);
     for (uint32_t p = 0; p < npix; ++p)
         dimg[p] = make_float4(dloss_dimage[3ull * p], dloss_dimage[3ull * p + 1], dloss_dimage[3ull * p + 2], 0.0f);
     if ((rc = begin_call(c, false))) return rc;
     WF_CUDA(h2d(c, c->dimage.p, dimg.data(), dimg.size() * sizeof(float4)));
     WF_CUDA(cudaMemsetAsync(c->g_albedo.p, 0, (uint64_t)replicas * ntri * sizeof(float4), c->stream));
-    WF_CUDA(cudaMemsetAsync(c->g_emission.p, 0, std::max<uint64_t>(ninst, 1) * sizeof(float), c->stream));
     WF_CUDA(cudaMemsetAsync(c->g_em_rep.p, 0, 32ull * std::max<uint64_t>(ninst, 1) * sizeof(float), c->stream));
-    const uint32_t wave = o->wave_paths ? std::min(o->wave_paths, c->capacity) : c->capacity;
     Pass P = make_pass(c, s, o, frame_seed);
-    P.fused = false;   // the replay's shadow rays need their own launches (AdjConnectIO)
+    P.fused = false;   // the shadow rays' launches record what they find
     P.fuse_from = 0;
     P.cnt = false;
     P.tail_paths = 0;
-    P.B.ps_Lc = c->L_comp.p;   // both passes keep the radiance sums' rounding errors
+    P.B.ps_Lc = c->L_comp.p;   // the radiance sums' rounding errors
     AdjointRefs A{};
     A.g_em_rep = c->g_em_rep.p;
-    A.L_final_lo = c->L_final_lo.p;
+    A.L_final_lo = c->L_comp.p;
     A.instances = (uint32_t)ninst;
-    A.L_final = c->L_final.p;
+    A.L_final = c->B.ps_L;
     A.dimage = c->dimage.p;
     A.g_albedo = c->g_albedo.p;
-    A.g_emission = c->g_emission.p;
     A.inv_spp = 1.0f / (float)o->spp;
     A.replicas = replicas;
     A.triangles = (uint32_t)ntri;
-    const AdjointRefs none{};
     for (const Wave& wv : plan_waves(o->spp, npix, wave)) {
-        // forward pass: each path's radiance, kept for the replay
-        if ((rc = run_wave(c, P, wv, 0, none, false))) return rc;
-        WF_CUDA(cudaMemcpyAsync(c->L_final.p, c->B.ps_L, (size_t)wv.k * wv.np * sizeof(float4),
-                                cudaMemcpyDeviceToDevice, c->stream));
-        WF_CUDA(cudaMemcpyAsync(c->L_final_lo.p, c->L_comp.p, (size_t)wv.k * wv.np * sizeof(float4),
-                                cudaMemcpyDeviceToDevice, c->stream));
-        // replay: the same paths from the same seeds, accumulating gradients
-        if ((rc = run_wave(c, P, wv, 0, A, false))) return rc;
+        // forward pass: each path's radiance and what its rays found
+        const uint64_t entries = depths * wv.k * wv.np;
+        P.B.tape_tuvp = reinterpret_cast<float4*>(c->tape.p);
+        P.B.tape_inst = reinterpret_cast<uint32_t*>(c->tape.p + 16 * entries);
+        P.B.tape_clear = c->tape.p + 20 * entries;
+        if (o->nee) WF_CUDA(cudaMemsetAsync(P.B.tape_clear, 0, entries, c->stream));
+        if ((rc = run_wave(c, P, wv, 0, false))) return rc;
+        // replay: the same paths from the same seeds and hits, accumulating gradients
+        {
+            StageTimer t(c, P.prof, ST_SHADE);
+            WF_CUDA(launch_replay(P.SH, P.B, P.W, A, c->stream));
+        }
+        c->launches++;
     }
     WF_CUDA(launch_reduce_replicas(c->g_albedo.p, (uint32_t)ntri, replicas, c->stream));
     c->launches++;
     std::vector<float4> ga(ntri);
-    std::vector<float> ge(ninst), gr(32ull * ninst);
+    std::vector<float> gr(32ull * ninst);
     WF_CUDA(d2h(c, ga.data(), c->g_albedo.p, ntri * sizeof(float4)));
     if (ninst) {
-        WF_CUDA(d2h(c, ge.data(), c->g_emission.p, ninst * sizeof(float)));
         WF_CUDA(d2h(c, gr.data(), c->g_em_rep.p, gr.size() * sizeof(float)));
     }
     if ((rc = end_call(c))) return rc;
@@ -1762,9 +1771,9 @@ int wf_adjoint(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
         d_albedo[3 * t + 2] = ga[t].z;
     }
     for (uint64_t i = 0; i < ninst; ++i) {
-        float e = ge[i];
-        for (uint32_t r = 0; r < 32; ++r) e = e + gr[(size_t)r * ninst + i];
-        d_emission[i] = e;
+        double e = 0.0;
+        for (uint32_t r = 0; r < 32; ++r) e = e + (double)gr[(size_t)r * ninst + i];
+        d_emission[i] = (float)e;
     }
     c->stats.paths = (uint64_t)npix * o->spp;
     return take_status(c);

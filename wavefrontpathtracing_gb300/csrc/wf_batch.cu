@@ -225,7 +225,7 @@ template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_bshade(ShadeRefs SH, const BatchScene* sc, BatchQueues Q, BatchCtl* c,
                                                   int cur) {
     const uint32_t n = c->count[cur];
-    const AdjointRefs none = {nullptr, nullptr, nullptr, nullptr, 0.0f, 1u, 0u};
+    const AdjointRefs none = {};
     const float4* const qo = cur ? Q.qo[1] : Q.qo[0];
     const float4* const qd = cur ? Q.qd[1] : Q.qd[0];
     const float4* const qT = cur ? Q.qT[1] : Q.qT[0];

@@ -26,8 +26,8 @@ struct ShadeRefs {
     uint32_t* status;
 };
 
-// Path-replay adjoint (null pointers in a forward pass).  The replay traces
-// the same paths as the forward pass; every path contribution is the product
+// Path-replay adjoint (null pointers in a forward pass).  The replay goes along
+// the paths of the forward pass; every path contribution is the product
 // of the Lambert albedos along the path and the emitter strength, so a vertex
 // on scene triangle t adds w * L / albedo(t) and the emitter adds w . L / strength,
 // with L the path's radiance from the forward pass and w = dloss/dimage / spp.
@@ -35,12 +35,11 @@ struct AdjointRefs {
     const float4* L_final;        // per path: radiance of the forward pass
     const float4* dimage;         // per pixel: dloss/d(average radiance)
     float4* g_albedo;             // replicas x scene triangles (atomic adds to x, y, z)
-    float* g_emission;            // per instance
     float inv_spp;
     uint32_t replicas;            // power of two; a warp adds into replica (block ^ warp) % replicas
     uint32_t triangles;
     const float4* L_final_lo;     // per path: the forward pass's ps_Lc (L_final + L_final_lo = the exact sum)
-    float* g_em_rep;              // shadow rays' emitter gradients: 32 replicas x instances
+    float* g_em_rep;              // emitter gradients: 32 replicas x instances
     uint32_t instances;
 };
 
@@ -59,7 +58,12 @@ struct RenderBuffers {
     float4* ps_T;         // {throughput rgb, pdf of the last BSDF sample}
     uint32_t* ps_flags;   // path flags
     float4* ps_L;         // path radiance (rgb), summed from zero
-    float4* ps_Lc;        // wf_adjoint's passes only (else null): the rounding errors of ps_L's additions
+    float4* ps_Lc;        // wf_adjoint's forward pass only (else null): the rounding errors of ps_L's additions
+    // wf_adjoint's forward pass only: what its rays found, per depth and path
+    // (entry depth * npaths + path), for the replay
+    float4* tape_tuvp;
+    uint32_t* tape_inst;
+    uint8_t* tape_clear;  // 1: the event's shadow ray was unoccluded (next-event estimation only)
     float4* s_o[2];       // shadow {origin, tmax}, by depth parity (connect at depth d
     float4* s_d[2];       // shadow {direction, path id}   runs while shade at d + 1
     float4* s_c[2];       // shadow {contribution rgb, -}  fills the other buffer)
@@ -117,19 +121,13 @@ cudaError_t launch_extend(const SceneRefs& S, const RenderBuffers& B, uint32_t d
 cudaError_t launch_extend_camera(const SceneRefs& S, const RenderBuffers& B, const WaveParams& W, bool count,
                                  unsigned long long* total, cudaStream_t stream);
 cudaError_t launch_shade(const ShadeRefs& SH, const RenderBuffers& B, const WaveParams& W, uint32_t depth,
-                         uint32_t max_rays, const AdjointRefs& A, cudaStream_t stream);
-// The adjoint replay's shadow rays (wf_adjoint with next-event estimation):
-// each unoccluded ray's contribution is linear in its emitter's strength.
-struct AdjConnect {
-    const float4* dimage;   // per pixel: dloss/d(average radiance)
-    const float4* sinst;    // shading rows (row 5 .w = emissive strength)
-    float* g_rep;           // 32 replicas x ninst emitter gradients (replica = queue slot % 32)
-    uint32_t ninst, pix0, nsamples;
-    float inv_spp;
-};
-cudaError_t launch_connect(const SceneRefs& S, const RenderBuffers& B, uint32_t depth, uint32_t max_rays,
-                           bool count, unsigned long long* total, cudaStream_t stream,
-                           const AdjConnect* adj = nullptr);
+                         uint32_t max_rays, cudaStream_t stream);
+// wf_adjoint: the wave's paths again, from the hits and visibilities that its
+// forward pass recorded (no ray is traced), accumulating A's gradients.
+cudaError_t launch_replay(const ShadeRefs& SH, const RenderBuffers& B, const WaveParams& W, const AdjointRefs& A,
+                          cudaStream_t stream);
+cudaError_t launch_connect(const SceneRefs& S, const RenderBuffers& B, uint32_t depth, uint32_t npaths, bool count,
+                           unsigned long long* total, cudaStream_t stream);
 // The shadow rays of depth - 1 and the extension rays of depth in one launch
 // (depth >= 1); totals[0] / totals[1] count the extension / shadow rays.
 cudaError_t launch_trace_pair(const SceneRefs& S, const RenderBuffers& B, uint32_t depth, unsigned long long* totals,

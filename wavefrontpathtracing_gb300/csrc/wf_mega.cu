@@ -30,7 +30,7 @@ __device__ __forceinline__ ShadeCtl make_ctl(const ShadeRefs& SH, const WavePara
 __device__ __forceinline__ float4 run_path(const SceneRefs& S, const ShadeRefs& SH, const ShadeCtl& K, uint32_t root,
                                            uint32_t pixel, uint32_t sample, uint32_t max_bounces, V3 ro, V3 rd,
                                            unsigned long long& n_ext, unsigned long long& n_con, bool& overflow) {
-    const AdjointRefs none = {nullptr, nullptr, nullptr, nullptr, 0.0f, 1u, 0u};
+    const AdjointRefs none = {};
     V3 T = mk(1.0f, 1.0f, 1.0f);
     float last_pdf = 0.0f;
     uint32_t flags = kFlagSpecular;

@@ -20,8 +20,8 @@ unsigned grid_for(uint32_t n) {
     return blocks ? blocks : 1u;
 }
 
-// Shade's block size and, for the plain variant, the resident blocks per SM
-// asked of the compiler (which caps its registers accordingly): 3 blocks of
+// Shade's block size and, for path tracing, the resident blocks per SM asked of
+// the compiler (which caps its registers accordingly): 3 blocks of
 // 256 (80 registers, 120 bytes of spills) measured 7 % faster per frame's
 // shade than 2 (126 registers) and 20 % faster than the one kernel for every
 // case (121 registers); 5 blocks of 128 (96 registers) in between.
@@ -33,14 +33,14 @@ unsigned grid_for(uint32_t n) {
 #endif
 constexpr int kShadeBlock = WF_SHADE_BLOCK;
 
-// PLAIN: path tracing without the adjoint's buffers or a debug view, the
-// render loop's usual case; the other variant serves every case, at 2
-// resident blocks (128 registers at most; left free it took 137, one block).
-template <bool PLAIN>
-__global__ void __launch_bounds__(kShadeBlock, PLAIN ? WF_SHADE_MIN_BLOCKS : 2)
-    k_shade(ShadeRefs SH, RenderBuffers B, WaveParams W, uint32_t depth, AdjointRefs A_in) {
-    const AdjointRefs A = PLAIN ? AdjointRefs{} : A_in;
-    if (PLAIN) B.ps_Lc = nullptr;
+// Path tracing (kPlain), path tracing that also keeps the radiance sums'
+// rounding errors and records the hits (kRecord, wf_adjoint's forward pass),
+// and the debug views (kViews, at 2 resident blocks).
+enum ShadeMode { kPlain, kRecord, kViews };
+template <int MODE>
+__global__ void __launch_bounds__(kShadeBlock, MODE == kViews ? 2 : WF_SHADE_MIN_BLOCKS)
+    k_shade(ShadeRefs SH, RenderBuffers B, WaveParams W, uint32_t depth) {
+    const AdjointRefs none = {};
     // depth 0 shades the camera paths of the wave in path order, their state
     // the one a path starts with (throughput 1, specular flag, no radiance),
     // so nothing is read but the hit; it also records the depth-0 count
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kShadeBlock, PLAIN ? WF_SHADE_MIN_BLOCKS : 2)
     K.frame_seed = W.frame_seed; K.max_bounces = W.max_bounces; K.nee = W.nee; K.rr_start = W.rr_start;
     K.cosine = W.cosine; K.env_strength = W.env_strength; K.env0 = W.env[0]; K.env1 = W.env[1]; K.env2 = W.env[2];
     K.lights = SH.lights; K.light_count = SH.light_count; K.light_total = SH.light_total;
-    K.env_tex = W.env_tex; K.view_mode = PLAIN ? 0u : W.view_mode; K.far_plane = W.far_plane;
+    K.env_tex = W.env_tex; K.view_mode = MODE == kViews ? W.view_mode : 0u; K.far_plane = W.far_plane;
     // shadow queue of this depth's parity (selects, not a dynamic index into the parameter)
     float4* const s_o = cur ? B.s_o[1] : B.s_o[0];
     float4* const s_d = cur ? B.s_d[1] : B.s_d[0];
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kShadeBlock, PLAIN ? WF_SHADE_MIN_BLOCKS : 2)
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t i = base + threadIdx.x;
         ShadeOut o;
-        o.enqueue = false; o.shadow = false; o.em_key = kInvalid; o.em_val = 0.0f;
+        o.enqueue = false; o.shadow = false;
         uint32_t path = 0;
         if (i < n) {
             ShadeIn in;
@@ -86,18 +86,16 @@ __global__ void __launch_bounds__(kShadeBlock, PLAIN ? WF_SHADE_MIN_BLOCKS : 2)
             in.inst = B.h_inst[i];
             in.sample = W.s0 + path % W.nsamples;
             in.depth = depth;
-            in.Lb = mk(0.0f, 0.0f, 0.0f);
-            in.Lb_lo = in.Lb;
-            if (A.g_albedo && depth) {
-                in.Lb = xyz(B.ps_L[path]);
-                in.Lb_lo = xyz(B.ps_Lc[path]);
+            if (MODE == kRecord) {
+                const size_t at = (size_t)depth * W.npaths + path;
+                B.tape_tuvp[at] = in.tuvp;
+                B.tape_inst[at] = in.inst;
             }
-            shade_one(SH, K, in, A, path, in.pixel, o);
+            shade_one(SH, K, in, none, 0u, 0u, o);
             if (o.has_add || depth == 0) {
                 // the path's radiance starts at zero here
                 float4 acc = depth ? B.ps_L[path] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (B.ps_Lc) {
-                    // the adjoint's passes also keep the additions' rounding errors
+                if (MODE == kRecord) {
                     float4 lc = depth ? B.ps_Lc[path] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     if (o.has_add) {
                         float e;
@@ -114,7 +112,6 @@ __global__ void __launch_bounds__(kShadeBlock, PLAIN ? WF_SHADE_MIN_BLOCKS : 2)
                 B.ps_L[path] = acc;
             }
         }
-        if (A.g_emission) warp_add_by_key(A.g_emission, o.em_key, o.em_val);
         const uint32_t slot = warp_append(&B.counts[depth + 1], o.enqueue);
         if (o.enqueue && in_bounds(slot, B.capacity, B.status)) {
             B.q_o[nxt][slot] = make_float4(o.org.x, o.org.y, o.org.z, __uint_as_float(o.flags & kFlagInside));
@@ -130,6 +127,78 @@ __global__ void __launch_bounds__(kShadeBlock, PLAIN ? WF_SHADE_MIN_BLOCKS : 2)
             s_c[sslot] = make_float4(o.contrib.x, o.contrib.y, o.contrib.z, __uint_as_float(o.light_inst));
         }
     }
+}
+
+// The adjoint's replay, one path per thread: every event of the path is shaded
+// again from the hit that the forward pass recorded, so no ray is traced and no
+// queue written; the path's state and its radiance so far (with its rounding
+// errors) stay in registers, summed in the forward pass's order.  The gradients
+// go out as shade_one's atomics, the emitters' into 32 replicas (a shadow ray's
+// contribution by path, the emitter a path ends at once per warp).
+//
+// Bound by the gathers of shade_one and the albedo atomics.  A 512x512 x 64
+// sample adjoint of depth 6 took 70.6 ms with a replay that traced every ray
+// again through the staged launches, 39.2 ms so (blocks of 256, 2 / 3 resident:
+// 39.3 / 39.4; 128, 7 resident: 39.3).
+constexpr int kReplayBlock = 128, kReplayMinBlocks = 5;
+__global__ void __launch_bounds__(kReplayBlock, kReplayMinBlocks)
+    k_replay(ShadeRefs SH, RenderBuffers B, WaveParams W, AdjointRefs A) {
+    const uint32_t path = blockIdx.x * kReplayBlock + threadIdx.x;
+    ShadeCtl K;
+    K.frame_seed = W.frame_seed; K.max_bounces = W.max_bounces; K.nee = W.nee; K.rr_start = W.rr_start;
+    K.cosine = W.cosine; K.env_strength = W.env_strength; K.env0 = W.env[0]; K.env1 = W.env[1]; K.env2 = W.env[2];
+    K.lights = SH.lights; K.light_count = SH.light_count; K.light_total = SH.light_total;
+    K.env_tex = W.env_tex; K.view_mode = 0u; K.far_plane = W.far_plane;
+    uint32_t em_key = kInvalid;
+    float em_val = 0.0f;
+    if (path < W.npaths) {
+        ShadeIn in;
+        in.pixel = W.pix0 + path / W.nsamples;
+        in.sample = W.s0 + path % W.nsamples;
+        V3 ro;
+        primary_ray(W, in.pixel % W.width, in.pixel / W.width, ro, in.rd);
+        in.T = mk(1.0f, 1.0f, 1.0f);
+        in.last_pdf = 0.0f;
+        in.flags = kFlagSpecular;
+        in.Lb = mk(0.0f, 0.0f, 0.0f);
+        in.Lb_lo = in.Lb;
+        auto gather = [&](V3 c) {
+            float e;
+            in.Lb.x = two_sum(in.Lb.x, c.x, e); in.Lb_lo.x = in.Lb_lo.x + e;
+            in.Lb.y = two_sum(in.Lb.y, c.y, e); in.Lb_lo.y = in.Lb_lo.y + e;
+            in.Lb.z = two_sum(in.Lb.z, c.z, e); in.Lb_lo.z = in.Lb_lo.z + e;
+        };
+        for (uint32_t depth = 0; depth <= W.max_bounces; ++depth) {
+            const size_t at = (size_t)depth * W.npaths + path;
+            in.tuvp = B.tape_tuvp[at];
+            in.inst = B.tape_inst[at];
+            in.depth = depth;
+            ShadeOut o;
+            shade_one(SH, K, in, A, path, in.pixel, o);
+            if (o.has_add) gather(o.add);
+            if (o.em_key != kInvalid) { em_key = o.em_key; em_val = o.em_val; }   // the path ends at an emitter
+            if (o.shadow && B.tape_clear[at]) {
+                gather(o.contrib);
+                // linear in the emitter's strength
+                if (in_bounds(o.light_inst, A.instances, B.status)) {
+                    const float strength = SH.sinst[(size_t)kInstRows * o.light_inst + 5].w;
+                    if (strength != 0.0f) {
+                        const float4 g = A.dimage[in.pixel];
+                        const float v = (g.x * A.inv_spp) * o.contrib.x + (g.y * A.inv_spp) * o.contrib.y +
+                                        (g.z * A.inv_spp) * o.contrib.z;
+                        atomicAdd(&A.g_em_rep[(size_t)(path & 31u) * A.instances + o.light_inst], v / strength);
+                    }
+                }
+            }
+            if (!o.enqueue) break;
+            in.rd = o.dir;
+            in.T = o.T;
+            in.last_pdf = o.pdf;
+            in.flags = o.flags;
+        }
+    }
+    const uint32_t rep = (blockIdx.x * (kReplayBlock / 32) + (threadIdx.x >> 5)) & 31u;
+    warp_add_by_key(A.g_em_rep + (size_t)rep * A.instances, em_key, em_val);
 }
 
 // post_process.hlsl:25-72 with accumulate on: average, NaN/Inf -> magenta,
@@ -197,14 +266,20 @@ __global__ void k_reduce_replicas(float4* g, uint32_t triangles, uint32_t replic
 }  // namespace
 
 cudaError_t launch_shade(const ShadeRefs& SH, const RenderBuffers& B, const WaveParams& W, uint32_t depth,
-                         uint32_t max_rays, const AdjointRefs& A, cudaStream_t stream) {
+                         uint32_t max_rays, cudaStream_t stream) {
     unsigned blocks = (max_rays + kShadeBlock - 1) / kShadeBlock;
     const unsigned cap = (unsigned)sm_count() * 8u * (256u / kShadeBlock);
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
-    const bool plain = !A.g_albedo && !A.g_emission && !B.ps_Lc && W.view_mode == 0u;
-    if (plain) k_shade<true><<<blocks, kShadeBlock, 0, stream>>>(SH, B, W, depth, A);
-    else k_shade<false><<<blocks, kShadeBlock, 0, stream>>>(SH, B, W, depth, A);
+    if (B.ps_Lc) k_shade<kRecord><<<blocks, kShadeBlock, 0, stream>>>(SH, B, W, depth);
+    else if (W.view_mode == 0u) k_shade<kPlain><<<blocks, kShadeBlock, 0, stream>>>(SH, B, W, depth);
+    else k_shade<kViews><<<blocks, kShadeBlock, 0, stream>>>(SH, B, W, depth);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_replay(const ShadeRefs& SH, const RenderBuffers& B, const WaveParams& W, const AdjointRefs& A,
+                          cudaStream_t stream) {
+    k_replay<<<(W.npaths + kReplayBlock - 1) / kReplayBlock, kReplayBlock, 0, stream>>>(SH, B, W, A);
     return cudaGetLastError();
 }
 

@@ -224,7 +224,7 @@ __device__ __forceinline__ void shade_one(const ShadeRefs& SH, const ShadeCtl& K
         }
         o.add = mk((T.x * le.x) * w, (T.y * le.y) * w, (T.z * le.z) * w);
         o.has_add = true;
-        if (A.g_emission && me.w != 0.0f) {
+        if (A.g_em_rep && me.w != 0.0f) {
             // the contribution is linear in this emitter's strength
             const float4 g = A.dimage[adj_pixel];
             const float gl = (g.x * A.inv_spp) * o.add.x + (g.y * A.inv_spp) * o.add.y + (g.z * A.inv_spp) * o.add.z;
