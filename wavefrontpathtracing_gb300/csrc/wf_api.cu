@@ -1516,6 +1516,8 @@ int run_wave(wf_ctx* c, Pass& P, const Wave& wv, uint32_t sample_base, bool reso
     W.pix0 = wv.p0;
     W.np = wv.np;
     W.npaths = wv.k * wv.np;
+    // the fetch counters count every path's own camera ray
+    W.camera_share = P.cnt ? 1u : W.nsamples;
     WF_CUDA(cudaMemsetAsync(B.counts, 0, 4 * kMaxDepth * sizeof(uint32_t), c->stream));
     if (P.mega) {
         // pathtracer.hlsl: every bounce of a path in one thread

@@ -86,9 +86,11 @@ struct WaveParams {
     float dim_x, dim_y;         // view_t.render_dim (uv of the primary ray)
     // A wave holds samples [s0, s0 + nsamples) of pixels [pix0, pix0 + np),
     // pixel-major: path p is sample s0 + p % nsamples of pixel pix0 + p / nsamples
-    // (npaths = nsamples * np), so the identical camera rays of a pixel's
-    // samples share a warp and traverse in lockstep.
+    // (npaths = nsamples * np), so a pixel's samples share a warp.
     uint32_t pix0, np, s0, nsamples, npaths;
+    // paths that share a camera ray: nsamples (it is traced once per pixel and
+    // its hit lies at entry p / nsamples), or 1 (every path's own is traced)
+    uint32_t camera_share;
     uint32_t frame_seed;
     uint32_t max_bounces, nee, rr_start, cosine;
     float env_strength;

@@ -82,8 +82,9 @@ __global__ void __launch_bounds__(kShadeBlock, MODE == kViews ? 2 : WF_SHADE_MIN
                 in.last_pdf = T4.w;
                 in.flags = B.ps_flags[path];
             }
-            in.tuvp = B.h_tuvp[i];
-            in.inst = B.h_inst[i];
+            const uint32_t hit = depth ? i : i / W.camera_share;
+            in.tuvp = B.h_tuvp[hit];
+            in.inst = B.h_inst[hit];
             in.sample = W.s0 + path % W.nsamples;
             in.depth = depth;
             if (MODE == kRecord) {

@@ -80,6 +80,17 @@ struct ChainIO<IO, std::void_t<decltype(IO::kChain)>> : std::true_type {};
 // running it for 2 / 4 / 8 / 16 ended lanes at a time measured 370 / 305 / 255 /
 // 247 us per 256x256 box frame against 235.
 
+// The paths that n rays of a source stand for, as the ray counts count them.
+template <class IO, class = void>
+struct SharedIO : std::false_type {};
+template <class IO>
+struct SharedIO<IO, std::void_t<decltype(std::declval<const IO&>().paths_of(0u))>> : std::true_type {};
+template <class IO>
+__device__ __forceinline__ uint32_t paths_of(const IO& io, uint32_t n) {
+    if constexpr (SharedIO<IO>::value) return io.paths_of(n);
+    else return n;
+}
+
 struct AosIO {
     const float4* rays;   // RayDesc2
     uint32_t* hits;       // hit_result_t
@@ -640,7 +651,7 @@ __global__ void __launch_bounds__(kTraceBlock, LAY ? WF_TRACE_QB_MIN_BLOCKS : WF
                                                   uint32_t* fetch, uint32_t* status, Counters* counters,
                                                   unsigned long long* total) {
     const uint32_t n = count_ptr ? *count_ptr : count;
-    if (total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(total, (unsigned long long)n);
+    if (total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(total, (unsigned long long)paths_of(io, n));
     LocalCounters c = {0, 0, 0, 0};
     bool overflow = false;
     trace_persistent<ANY, COUNT, LAY>(S, io, n, fetch, c, overflow);
