@@ -130,7 +130,7 @@ struct wf_ctx {
     DevBuf<TexRef> tex_table;               // entry 0 unused
 
     // device scene
-    DevBuf<float4> tnodes, tinst, sinst;
+    DevBuf<float4> tnodes, tpairs, tinst, sinst;
     DevBuf<BlasRef> blas;
     DevBuf<const float4*> stri;
     DevBuf<LightTri> lights;
@@ -502,6 +502,7 @@ void release_buffers(wf_ctx* c) {
 SceneRefs scene_refs(wf_ctx* c) {
     SceneRefs S;
     S.tnodes = c->tnodes.p;
+    S.tpairs = c->tpairs.p;
     S.tinst = c->tinst.p;
     S.blas = c->blas.p;
     S.inst_count = (uint32_t)c->scene_bi.size();
@@ -988,7 +989,7 @@ int wf_destroy(wf_ctx* c) {
     for (Texture& t : c->textures) dev_free(t.d);
     c->tex_table.release();
     release_buffers(c);
-    c->tnodes.release(); c->tinst.release(); c->sinst.release(); c->blas.release(); c->stri.release();
+    c->tnodes.release(); c->tpairs.release(); c->tinst.release(); c->sinst.release(); c->blas.release(); c->stri.release();
     c->lights.release(); c->aabbs.release(); c->tlas_scratch.release();
     c->tri_albedo.release(); c->inst_tri_offset.release(); c->dimage.release();
     c->g_albedo.release(); c->g_em_rep.release(); c->L_comp.release(); c->tape.release();
@@ -1292,7 +1293,7 @@ int wf_scene_end(wf_ctx* c) {
         c->scene_bi[i] = in.bi;
         instance_rows(in, &ti[4ull * i], &si[(size_t)kInstRows * i], &aabbs[6ull * i]);
     }
-    if ((rc = c->tnodes.reserve(2ull * std::max<uint32_t>(2 * n, 1))) || (rc = c->tinst.reserve(ti.size())) ||
+    if ((rc = c->tnodes.reserve(2ull * std::max<uint32_t>(2 * n, 1))) || (rc = c->tpairs.reserve(8ull * n)) || (rc = c->tinst.reserve(ti.size())) ||
         (rc = c->sinst.reserve(si.size())) || (rc = c->aabbs.reserve(aabbs.size())) ||
         (rc = c->tlas_scratch.reserve(tlas_scratch_words(n, c->tlas_metric))))
         return rc;
@@ -1316,7 +1317,8 @@ int wf_scene_end(wf_ctx* c) {
             WF_CUDA(h2d(c, c->aabbs.p, aabbs.data(), aabbs.size() * 4));
         }
         WF_CUDA(launch_tlas_build(c->aabbs.p, n, c->tnodes.p, c->tlas_scratch.p, c->tlas_metric, c->stream));
-        c->launches++;
+        WF_CUDA(launch_tlas_pairs(c->tnodes.p, 2 * n, c->tpairs.p, c->stream));
+        c->launches += 2;
     }
     // emitter table (every triangle of every emissive instance, world space)
     std::vector<LightTri> lt;

@@ -416,7 +416,7 @@ struct wf_batch {
     uint32_t nscenes = 0, total_paths = 0, total_pixels = 0, total_inst = 0;
     std::vector<uint32_t> light_off, light_cnt, roots;
     std::vector<float> light_total;
-    DBuf<float4> tnodes, tinst, sinst;
+    DBuf<float4> tnodes, tpairs, tinst, sinst;
     DBuf<float> aabbs;
     DBuf<uint32_t> tlas_scratch, d_roots, d_pbase, d_pixbase;
     DBuf<LightTri> lights;
@@ -543,7 +543,7 @@ int build_tables(wf_batch* b) {
         pbase[s + 1] = pbase[s] + H.width * H.height * H.spp;
         pixbase[s + 1] = pixbase[s] + H.width * H.height;
     }
-    if ((rc = b->tnodes.reserve(4ull * std::max<uint32_t>(ni, 1))) || (rc = b->tinst.reserve(ti.size())) ||
+    if ((rc = b->tnodes.reserve(4ull * std::max<uint32_t>(ni, 1))) || (rc = b->tpairs.reserve(8ull * ni)) || (rc = b->tinst.reserve(ti.size())) ||
         (rc = b->sinst.reserve(si.size())) || (rc = b->aabbs.reserve(ab.size())) ||
         (rc = b->tlas_scratch.reserve(tlas_scratch_words(ni, ctx_tlas_metric(c)))) || (rc = b->lights.reserve(lt.size())) ||
         (rc = b->d_roots.reserve(ns)) || (rc = b->d_pbase.reserve(ns + 1)) || (rc = b->d_pixbase.reserve(ns + 1)) ||
@@ -568,6 +568,7 @@ int build_tables(wf_batch* b) {
         k_tlas_rebase<<<(2 * n + 127) / 128, 128, 0, st>>>(nodes, 2 * n, 2 * ibase[s], ibase[s]);
         BCUDA(cudaGetLastError());
     }
+    BCUDA(launch_tlas_pairs(b->tnodes.p, 2 * ni, b->tpairs.p, st));
     BCUDA(cudaStreamSynchronize(st));
     b->tables_ready = true;
     drop_graph(b);
@@ -655,6 +656,7 @@ int enqueue_iteration(wf_batch* b, int k, bool join_prev, bool join_self, cudaGr
     const BatchQueues Q = queues(b);
     SceneRefs S;
     S.tnodes = b->tnodes.p;
+    S.tpairs = b->tpairs.p;
     S.tinst = b->tinst.p;
     S.blas = b->blas.p;
     S.inst_count = b->total_inst;
@@ -891,7 +893,7 @@ int wf_batch_destroy(wf_batch* b) {
     ctx_use_device(b->ctx);
     cudaStreamSynchronize(ctx_stream(b->ctx));
     drop_graph(b);
-    b->tnodes.release(); b->tinst.release(); b->sinst.release(); b->aabbs.release();
+    b->tnodes.release(); b->tpairs.release(); b->tinst.release(); b->sinst.release(); b->aabbs.release();
     b->tlas_scratch.release(); b->d_roots.release(); b->d_pbase.release(); b->d_pixbase.release();
     b->lights.release(); b->blas.release(); b->stri.release(); b->d_scenes.release();
     b->out_L.release(); b->image.release();

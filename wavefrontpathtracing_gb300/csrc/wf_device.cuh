@@ -25,6 +25,10 @@ namespace wf {
 //           storing them changes no result and removes the index indirection.
 // TLAS:
 //   tnodes: the reference's 32-byte tlas_node_t verbatim.
+//   tpairs: entry k = the two children of interior node k, 4 x float4 as a BLAS
+//           child pair {min.xyz, first} {max.xyz, count}: first = 2 * the child's
+//           index and count = 0 for an interior child, its instance and 1 for a
+//           leaf; made from tnodes, so that one step serves both levels.
 //   tinst : 4 x float4 per instance: world_to_local columns m[0..2], m[4..6],
 //           m[8..10], m[12..14] (the only entries the transform reads), with
 //           the mesh id in the first .w.
@@ -49,6 +53,7 @@ struct BlasRef {
 
 struct SceneRefs {
     const float4* tnodes;      // TLAS nodes
+    const float4* tpairs;      // per interior TLAS node: its two children as a BLAS child pair
     const float4* tinst;       // TLAS instances
     const BlasRef* blas;       // indexed by mesh id
     uint32_t inst_count;

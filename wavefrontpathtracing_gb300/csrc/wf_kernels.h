@@ -175,6 +175,9 @@ cudaError_t launch_instance_bounds(const float4* sinst, uint32_t rows, uint32_t 
 cudaError_t launch_tlas_build(const float* aabbs /* 6 floats per instance */, uint32_t n, float4* nodes,
                               uint32_t* scratch, uint32_t metric, cudaStream_t stream);
 
+// The child pairs of count nodes (SceneRefs.tpairs, 4 float4 per node).
+cudaError_t launch_tlas_pairs(const float4* nodes, uint32_t count, float4* pairs, cudaStream_t stream);
+
 int sm_count();
 // Device allocations of the library go through these: they enforce the
 // process-wide limit set by wf_set_device_memory_limit (an allocation past it

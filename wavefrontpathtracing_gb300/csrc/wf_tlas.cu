@@ -1405,6 +1405,27 @@ cudaError_t launch_instance_bounds(const float4* sinst, uint32_t rows, uint32_t 
     return cudaGetLastError();
 }
 
+namespace {
+__global__ void k_tlas_pairs(const float4* __restrict__ nodes, uint32_t count, float4* __restrict__ pairs) {
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, k = q >> 1;
+    if (k >= count) return;
+    const uint32_t lr = __float_as_uint(nodes[2ull * k].w);
+    if (lr == 0u) return;   // a leaf
+    const uint32_t c = (q & 1u) ? lr & 0xFFFFu : lr >> 16;
+    if (c >= count) return;
+    const float4 a = nodes[2ull * c], b = nodes[2ull * c + 1];
+    const bool leaf = __float_as_uint(a.w) == 0u;
+    pairs[2ull * q] = make_float4(a.x, a.y, a.z, leaf ? b.w : __uint_as_float(2u * c));
+    pairs[2ull * q + 1] = make_float4(b.x, b.y, b.z, __uint_as_float(leaf ? 1u : 0u));
+}
+}  // namespace
+
+cudaError_t launch_tlas_pairs(const float4* nodes, uint32_t count, float4* pairs, cudaStream_t stream) {
+    if (count == 0) return cudaSuccess;
+    k_tlas_pairs<<<(2 * count + 127) / 128, 128, 0, stream>>>(nodes, count, pairs);
+    return cudaGetLastError();
+}
+
 size_t tlas_scratch_words(uint32_t n, uint32_t metric) {
     if (metric == 2) return (n <= kPlocSmemMax) ? 8 : ploc_bytes(n, pow2_at_least(n ? n : 1)) / 4 + 8;
     if (metric == 3) return (n <= kSweepSmemMax) ? 8 : sweep_words(n, pow2_at_least(n ? n : 1)) + 8;
