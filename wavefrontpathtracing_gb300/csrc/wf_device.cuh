@@ -225,6 +225,31 @@ __device__ __forceinline__ float slab(V3 bmn, V3 bmx, V3 o, V3 inv, float t) {
     return (tmax >= tmin && tmin < t && tmax > 0.0f) ? tmin : FLT_MAX;
 }
 
+// slab for a node's two float4 as stored, with the x and y planes' subtractions
+// and products as packed pairs (adjacent registers of one load; b - o is b + (-o)
+// exactly): the same tmin in a third fewer floating-point instructions; returns
+// whether the box is entered before t.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 add_mul2(float x, float y, unsigned long long add, unsigned long long mul) {
+    float2 r;
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%2, %3};\n\tadd.rn.f32x2 a, a, %4;\n\tmul.rn.f32x2 b, a, %5;\n\t"
+        "mov.b64 {%0, %1}, b;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(x), "f"(y), "l"(add), "l"(mul));
+    return r;
+}
+__device__ __forceinline__ bool slab_hit(float4 bmn, float4 bmx, V3 o, V3 inv, float t, float& tmin) {
+    const unsigned long long no = pack2(-o.x, -o.y), iv = pack2(inv.x, inv.y);
+    const float2 l = add_mul2(bmn.x, bmn.y, no, iv), h = add_mul2(bmx.x, bmx.y, no, iv);
+    const float tz1 = (bmn.z - o.z) * inv.z, tz2 = (bmx.z - o.z) * inv.z;
+    tmin = fmaxf(fmaxf(fminf(l.x, h.x), fminf(l.y, h.y)), fminf(tz1, tz2));
+    const float tmax = fminf(fminf(fmaxf(l.x, h.x), fmaxf(l.y, h.y)), fmaxf(tz1, tz2));
+    return tmax >= tmin && tmin < t && tmax > 0.0f;
+}
+
 // The slab test of the order-independent tie rule (closest-hit rays over the
 // quantized layout): a box entered at exactly the current t is still visited,
 // since it may hold an equal-t hit with a smaller (instance, primitive).

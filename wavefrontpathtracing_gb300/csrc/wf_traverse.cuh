@@ -56,8 +56,7 @@ constexpr int kTraceBlock = WF_TRACE_BLOCK;
 // reference.  Its top WF_TRACE_RING entries live in a shared-memory ring (slot
 // index % ring, one column per thread), the older ones in local memory; a
 // push into a full ring moves the ring's oldest entry to local memory, a pop
-// from an empty ring reads local memory.  WF_TRACE_RING 0 keeps the whole
-// stack in local memory.
+// from an empty ring reads local memory.
 #ifndef WF_TRACE_RING
 #define WF_TRACE_RING 8
 #endif
@@ -168,18 +167,20 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
     BlasRef B;
     B.nodes = nullptr; B.tris = nullptr;
     // stack: entries [0, sp); the TLAS level's are [0, tb) while inside an
-    // instance; [lo, sp) are in the ring, [0, lo) in local memory
+    // instance (tb = 0 outside); [lo, sp) are in the ring, [0, lo) in local memory
     int sp = 0, lo = 0, tb = 0;
     uint2 deep[2 * kStack];
-#if WF_TRACE_RING > 0
     __shared__ uint2 ring[WF_TRACE_RING][kTraceBlock];
-    auto stack_push = [&](uint2 e) {
+    // false: the level's 64 entries are taken
+    auto stack_push = [&](uint2 e) -> bool {
+        if (sp - tb == kStack) return false;
         if (sp - lo == WF_TRACE_RING) {
             deep[lo] = ring[lo % WF_TRACE_RING][col];
             lo++;
         }
         ring[sp % WF_TRACE_RING][col] = e;
         sp++;
+        return true;
     };
     auto stack_pop = [&]() -> uint2 {
         sp--;
@@ -187,10 +188,6 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
         lo = sp;
         return deep[sp];
     };
-#else
-    auto stack_push = [&](uint2 e) { deep[sp++] = e; };
-    auto stack_pop = [&]() -> uint2 { return deep[--sp]; };
-#endif
     auto hit_record = [&]() {
         Hit h;
         h.inst = s_inst[col]; h.prim = s_prim[col]; h.t = s_t[col]; h.u = s_u[col]; h.v = s_v[col];
@@ -229,7 +226,7 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
             level = 0; nb = S.tpairs;
             w0 = leaf ? __float_as_uint(n1.w) : 2u * root;
             w1 = leaf ? 1u : 0u;
-            sp = 0; lo = 0;
+            sp = 0; lo = 0; tb = 0;
         }
         return !miss;
     };
@@ -411,11 +408,9 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
 #pragma unroll
                     for (int i = 3; i >= 1; --i) {
                         if (d[i] != FLT_MAX && !finish) {
-                            if (sp - tb == kStack) {
+                            if (!stack_push(e[i])) {
                                 clear_hit();
                                 finish = true; ok = false; overflow = true;
-                            } else {
-                                stack_push(e[i]);
                             }
                         }
                     }
@@ -430,26 +425,25 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
             } else {
                 const float4 a0 = ldg4(pa), a1 = ldg4(pa + 1), b0 = ldg4(pa + 2), b1 = ldg4(pa + 3);
                 if (COUNT) { if (level == 0u) cnt.tlas_nodes += 2; else cnt.blas_nodes += 2; }
-                const bool tie = QB && !any_ray;
-                float dl = tie ? slab_le(xyz(a0), xyz(a1), co, ci, ct) : slab(xyz(a0), xyz(a1), co, ci, ct);
-                float dr = tie ? slab_le(xyz(b0), xyz(b1), co, ci, ct) : slab(xyz(b0), xyz(b1), co, ci, ct);
-                uint2 L = make_uint2(__float_as_uint(a0.w), __float_as_uint(a1.w));
-                uint2 R = make_uint2(__float_as_uint(b0.w), __float_as_uint(b1.w));
-                if (dl > dr) {
-                    float td = dl; dl = dr; dr = td;
-                    uint2 tn = L; L = R; R = tn;
-                }
-                if (dl == FLT_MAX) {
-                    pop = true;
+                float dl, dr;
+                bool hl, hr;   // the children entered before the current hit
+                if (QB && !any_ray) {
+                    dl = slab_le(xyz(a0), xyz(a1), co, ci, ct); hl = dl != FLT_MAX;
+                    dr = slab_le(xyz(b0), xyz(b1), co, ci, ct); hr = dr != FLT_MAX;
                 } else {
-                    w0 = L.x; w1 = L.y;
-                    if (dr != FLT_MAX) {
-                        if ((level == 0u ? sp : sp - tb) == kStack) {
-                            clear_hit();
-                            finish = true; ok = false; overflow = true;
-                        } else {
-                            stack_push(R);
-                        }
+                    hl = slab_hit(a0, a1, co, ci, ct, dl);
+                    hr = slab_hit(b0, b1, co, ci, ct, dr);
+                }
+                // the nearer first, ties to the left
+                const bool right = hr && (!hl || dl > dr);
+                pop = !hl && !hr;
+                w0 = __float_as_uint(right ? b0.w : a0.w);
+                w1 = __float_as_uint(right ? b1.w : a1.w);
+                if (hl && hr) {
+                    const uint2 far = make_uint2(__float_as_uint(right ? a0.w : b0.w), __float_as_uint(right ? a1.w : b1.w));
+                    if (!stack_push(far)) {
+                        clear_hit();
+                        finish = true; ok = false; overflow = true;
                     }
                 }
             }
@@ -463,7 +457,7 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
                 } else {
                     // leave the instance: ray.t = ray_local.t (accelstruct.hlsl:146, 170-174)
                     if (hit_here) { s_inst[col] = ii; s_t[col] = ct; }
-                    level = 0; nb = S.tpairs;
+                    level = 0; nb = S.tpairs; tb = 0;
                     co = xyz(s_wo[col]); cd = xyz(s_wd[col]); ci = rcp(cd);
                 }
             }
