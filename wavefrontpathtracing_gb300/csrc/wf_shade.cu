@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(kShadeBlock, MODE == kViews ? 2 : WF_SHADE_MIN
 // sample adjoint of depth 6 took 70.6 ms with a replay that traced every ray
 // again through the staged launches, 39.2 ms so (blocks of 256, 2 / 3 resident:
 // 39.3 / 39.4; 128, 7 resident: 39.3).
+// (All with single-float albedo atomics and an earlier traversal loop; 29.2 ms now.)
 constexpr int kReplayBlock = 128, kReplayMinBlocks = 5;
 __global__ void __launch_bounds__(kReplayBlock, kReplayMinBlocks)
     k_replay(ShadeRefs SH, RenderBuffers B, WaveParams W, AdjointRefs A) {
