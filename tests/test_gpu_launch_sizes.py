@@ -8,7 +8,11 @@ nothing past the last ray.
 
 Waves of at most 65,536 paths without shadow rays run whole in one launch;
 their images and ray counts must equal the staged launches' (which profiled
-frames use) and the megakernel's, below, at and above that size."""
+frames use) and the megakernel's, below, at and above that size.
+
+Shade places a block's continuation and shadow rays in the queues by octant:
+around the block's size no ray may be lost or written twice, so images must
+equal the megakernel's."""
 import numpy as np
 import pytest
 
@@ -68,3 +72,17 @@ def test_whole_waves_equal_staged_launches(width, height, spp, bounces, rr, wave
         assert stats[0]["rays_extend"] == stats[k]["rays_extend"] and stats[0]["rays_connect"] == 0
     assert stats[0]["extend_rays_depth"] == stats[1]["extend_rays_depth"]
     assert (stats[0]["launches"] < stats[1]["launches"]) == ((wave or width * height * spp) <= 65536)
+
+
+@pytest.mark.parametrize("width,height,spp,bounces,wave", [
+    (1, 1, 1, 3, 0), (127, 1, 1, 3, 0), (128, 1, 1, 3, 0), (43, 1, 3, 3, 0), (61, 37, 2, 6, 0), (61, 37, 2, 6, 257),
+    (641, 359, 1, 2, 0)])
+def test_queues_hold_every_ray(width, height, spp, bounces, wave):
+    desc = scenes.mixed_box_scene(width, height)
+    kw = dict(max_bounces=bounces, spp=spp, nee=1, rr_start_depth=2, wave_paths=wave, frame_seed=11, accumulate=False)
+    with Renderer(width, height) as r:
+        load_scene_into(r, desc)
+        r.render(**kw)
+        image = r.read_image()
+        r.render(megakernel=True, **kw)
+        assert np.array_equal(image.view(np.uint32), r.read_image().view(np.uint32))

@@ -239,10 +239,12 @@ __global__ void __launch_bounds__(BLOCK) k_bshade(ShadeRefs SH, const BatchScene
     float4* const s_o = cur ? Q.s_o[1] : Q.s_o[0];
     float4* const s_d = cur ? Q.s_d[1] : Q.s_d[0];
     float4* const s_c = cur ? Q.s_c[1] : Q.s_c[0];
+    __shared__ BlockAppend<BLOCK> append;
     for (uint32_t base = blockIdx.x * BLOCK; base < n; base += gridDim.x * BLOCK) {
         const uint32_t i = base + threadIdx.x;
         ShadeOut o;
         o.enqueue = false; o.shadow = false;
+        o.dir = mk(0, 0, 0); o.sdir = mk(0, 0, 0);
         uint32_t scene = 0, depth = 0, pixel = 0, gidx = 0;
         float4 L4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (i < n) {
@@ -281,7 +283,8 @@ __global__ void __launch_bounds__(BLOCK) k_bshade(ShadeRefs SH, const BatchScene
                 if (in_bounds(gidx, Q.total_paths, Q.status)) Q.out_L[gidx] = L4;
             }
         }
-        const uint32_t slot = warp_append(ncount, o.enqueue);
+        const uint2 slots = append(ncount, o.enqueue, o.dir, shadow_tail, o.shadow, o.sdir);
+        const uint32_t slot = slots.x, sslot = slots.y;
         if (o.enqueue && in_bounds(slot, Q.capacity, Q.status)) {
             const uint32_t f = (o.flags & 0xFFu) | ((depth + 1u) << kDepthShift) | (scene << kSceneShift);
             no[slot] = make_float4(o.org.x, o.org.y, o.org.z, __uint_as_float(f));
@@ -289,7 +292,6 @@ __global__ void __launch_bounds__(BLOCK) k_bshade(ShadeRefs SH, const BatchScene
             nT[slot] = make_float4(o.T.x, o.T.y, o.T.z, o.pdf);
             nL[slot] = L4;
         }
-        const uint32_t sslot = warp_append(shadow_tail, o.shadow);
         if (o.shadow && in_bounds(sslot, Q.capacity, Q.status)) {
             const uint32_t target = o.enqueue ? slot : (kFinishedBit | gidx);
             s_o[sslot] = make_float4(o.spos.x, o.spos.y, o.spos.z, o.stmax);

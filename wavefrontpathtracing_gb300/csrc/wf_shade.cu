@@ -21,15 +21,16 @@ unsigned grid_for(uint32_t n) {
 }
 
 // Shade's block size and, for path tracing, the resident blocks per SM asked of
-// the compiler (which caps its registers accordingly): 3 blocks of
-// 256 (80 registers, 120 bytes of spills) measured 7 % faster per frame's
-// shade than 2 (126 registers) and 20 % faster than the one kernel for every
-// case (121 registers); 5 blocks of 128 (96 registers) in between.
+// the compiler (which caps its registers accordingly): 768 threads per SM (80
+// registers, some spills) measured 7 % faster per frame's shade than 512 (126
+// registers).  6 blocks of 128 rather than 3 of 256, whose barriers hold more
+// warps up: 613x377 textured frame 1.770 -> 1.758 ms, 1080p instanced frame 9.87
+// -> 9.85; 5 of 128: 1.786 and 9.98.
 #ifndef WF_SHADE_BLOCK
-#define WF_SHADE_BLOCK 256
+#define WF_SHADE_BLOCK 128
 #endif
 #ifndef WF_SHADE_MIN_BLOCKS
-#define WF_SHADE_MIN_BLOCKS 3
+#define WF_SHADE_MIN_BLOCKS 6
 #endif
 constexpr int kShadeBlock = WF_SHADE_BLOCK;
 
@@ -56,11 +57,13 @@ __global__ void __launch_bounds__(kShadeBlock, MODE == kViews ? 2 : WF_SHADE_MIN
     float4* const s_o = cur ? B.s_o[1] : B.s_o[0];
     float4* const s_d = cur ? B.s_d[1] : B.s_d[0];
     float4* const s_c = cur ? B.s_c[1] : B.s_c[0];
+    __shared__ BlockAppend<kShadeBlock> append;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t i = base + threadIdx.x;
         ShadeOut o;
         o.enqueue = false; o.shadow = false;
+        o.dir = mk(0, 0, 0); o.sdir = mk(0, 0, 0);
         uint32_t path = 0;
         if (i < n) {
             ShadeIn in;
@@ -113,7 +116,16 @@ __global__ void __launch_bounds__(kShadeBlock, MODE == kViews ? 2 : WF_SHADE_MIN
                 B.ps_L[path] = acc;
             }
         }
-        const uint32_t slot = warp_append(&B.counts[depth + 1], o.enqueue);
+        uint2 slots;
+        if (MODE == kPlain) {
+            slots = append(&B.counts[depth + 1], o.enqueue, o.dir, &B.counts[kMaxDepth + depth], o.shadow, o.sdir);
+        } else {
+            // the adjoint's tape is written by path, and loses more to a queue out
+            // of path order (33.0 -> 34.1 ms) than its rays gain
+            slots.x = warp_append(&B.counts[depth + 1], o.enqueue);
+            slots.y = warp_append(&B.counts[kMaxDepth + depth], o.shadow);
+        }
+        const uint32_t slot = slots.x, sslot = slots.y;
         if (o.enqueue && in_bounds(slot, B.capacity, B.status)) {
             B.q_o[nxt][slot] = make_float4(o.org.x, o.org.y, o.org.z, __uint_as_float(o.flags & kFlagInside));
             B.q_d[nxt][slot] = make_float4(o.dir.x, o.dir.y, o.dir.z, FLT_MAX);
@@ -121,7 +133,6 @@ __global__ void __launch_bounds__(kShadeBlock, MODE == kViews ? 2 : WF_SHADE_MIN
             B.ps_T[path] = make_float4(o.T.x, o.T.y, o.T.z, o.pdf);
             B.ps_flags[path] = o.flags;
         }
-        const uint32_t sslot = warp_append(&B.counts[kMaxDepth + depth], o.shadow);
         if (o.shadow && in_bounds(sslot, B.capacity, B.status)) {
             s_o[sslot] = make_float4(o.spos.x, o.spos.y, o.spos.z, o.stmax);
             s_d[sslot] = make_float4(o.sdir.x, o.sdir.y, o.sdir.z, __uint_as_float(path));

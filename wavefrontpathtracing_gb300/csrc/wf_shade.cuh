@@ -21,6 +21,63 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* tail, bool want) {
     return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
 }
 
+// Slot allocation for a block's continuation and shadow rays (a and b): one
+// atomicAdd per block and queue, and within the block's share the rays ordered
+// by the octant of their direction, so the warps that trace them later hold
+// rays that start close together and go the same way: 613x377 textured frame
+// 1.81 -> 1.76 ms, batch of 11 scenes 8.75 -> 8.58, 1080p instanced frame 9.93 ->
+// 9.85 (continuation rays only: 1.77, 8.60, 9.90).
+template <int BLOCK>
+struct BlockAppend {
+    static constexpr int kWarps = BLOCK / 32, kPer = kWarps * 8 / 32;   // counters a scanning lane holds
+    static_assert(kPer >= 1 && kWarps >= 2, "");
+    uint32_t n[2][8 * kWarps];   // [queue][octant, warp]: the warp's rays, then their first slot
+
+    static __device__ __forceinline__ uint32_t octant(V3 d) {
+        return (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
+    }
+    // the lanes of the warp that want a slot in octant k
+    static __device__ __forceinline__ unsigned lanes(const unsigned (&b)[4], uint32_t k) {
+        return b[3] & (k & 1u ? b[0] : ~b[0]) & (k & 2u ? b[1] : ~b[1]) & (k & 4u ? b[2] : ~b[2]);
+    }
+    // every thread of the block calls it
+    __device__ __forceinline__ uint2 operator()(uint32_t* tail_a, bool want_a, V3 dir_a, uint32_t* tail_b, bool want_b,
+                                                V3 dir_b) {
+        const unsigned FULL = 0xffffffffu;
+        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+        const uint32_t key[2] = {octant(dir_a), octant(dir_b)};
+        uint32_t rank[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const unsigned b[4] = {__ballot_sync(FULL, key[q] & 1u), __ballot_sync(FULL, key[q] & 2u),
+                                   __ballot_sync(FULL, key[q] & 4u), __ballot_sync(FULL, q ? want_b : want_a)};
+            if (lane < 8u) n[q][lane * kWarps + warp] = (uint32_t)__popc(lanes(b, lane));
+            rank[q] = (uint32_t)__popc(lanes(b, key[q]) & ((1u << lane) - 1u));
+        }
+        __syncthreads();
+        if (warp < 2u) {   // warp 0 places a's rays, warp 1 b's
+            uint32_t* const m = n[warp];
+            uint32_t c[kPer], sum = 0;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) { c[k] = m[lane * kPer + k]; sum += c[k]; }
+            uint32_t at = sum;
+#pragma unroll
+            for (uint32_t d = 1; d < 32u; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(FULL, at, d);
+                if (lane >= d) at += v;
+            }
+            const uint32_t total = __shfl_sync(FULL, at, 31);
+            uint32_t base = 0;
+            if (lane == 0u && total) base = atomicAdd(warp ? tail_b : tail_a, total);
+            at = __shfl_sync(FULL, base, 0) + at - sum;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) { m[lane * kPer + k] = at; at += c[k]; }
+        }
+        __syncthreads();
+        return make_uint2(n[0][key[0] * kWarps + warp] + rank[0], n[1][key[1] * kWarps + warp] + rank[1]);
+    }
+};
+
 // make_primary_ray (common.hlsl:182-195).
 template <class Cam>
 __device__ __forceinline__ void primary_ray(const Cam& W, uint32_t px, uint32_t py, V3& o, V3& d) {
