@@ -305,6 +305,13 @@ __device__ __forceinline__ bool tri_hit_tie(V3 v0, V3 e1, V3 e2, V3 o, V3 d, flo
 }
 
 __device__ __forceinline__ float4 ldg4(const float4* p) { return __ldg(p); }
+// Two consecutive float4 in one load, the first on a 32-byte boundary (as every
+// node, instance row and 4-wide node is: an even float4 of an allocation).
+__device__ __forceinline__ void ldg8(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(__cvta_generic_to_global(p)));
+}
 
 // ---------------------------------------------------------------- textures
 // Texture slots of material_t and the values of the reference's default

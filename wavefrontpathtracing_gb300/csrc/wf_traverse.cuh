@@ -36,7 +36,9 @@
 // 11.31 ms, 1.07, 370 us, 5.99 ms; several steps per iteration (one kind of
 // step per lane and iteration before) with the world ray's reciprocal kept
 // through an instance: 9.91 ms, 1.02, 316 us, 5.49 ms, and a whole-wave 256x256
-// frame 222 -> 172 us.
+// frame 222 -> 172 us; then nodes and instance rows in 32-byte loads, half the
+// requests: 9.53 ms, 1.02, 298 us, 4.46 ms (quantized and exact 4-wide: 6.02 ->
+// 6.01, 7.04 -> 6.07).
 #pragma once
 #include <type_traits>
 #include "wf_device.cuh"
@@ -238,7 +240,8 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
         bool miss = root == kInvalid;
         if (!miss && !in_bounds(root, S.tnode_count, S.status)) miss = true;
         if (!miss) {
-            const float4 n0 = ldg4(S.tnodes + 2ull * root), n1 = ldg4(S.tnodes + 2ull * root + 1);
+            float4 n0, n1;
+            ldg8(S.tnodes + 2ull * root, n0, n1);
             if (COUNT) cnt.tlas_nodes++;
             miss = ((QB && !any_ray) ? slab_le(xyz(n0), xyz(n1), co, ci, ct)
                                      : slab(xyz(n0), xyz(n1), co, ci, ct)) == FLT_MAX;
@@ -307,7 +310,9 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
                 w1 = 0u;
                 pop = true;
             } else {
-                const float4 c0 = ldg4(ip), c1 = ldg4(ip + 1), c2 = ldg4(ip + 2), c3 = ldg4(ip + 3);
+                float4 c0, c1, c2, c3;
+                ldg8(ip, c0, c1);
+                ldg8(ip + 2, c2, c3);
                 if (COUNT) cnt.instances++;
                 const uint32_t mesh = __float_as_uint(c0.w);
                 if (!in_bounds(mesh, S.mesh_count, S.status)) {
@@ -323,7 +328,8 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
                         w0 = 0u;
                         w1 = B.root_count;
                     } else {
-                        const float4 r0 = ldg4(B.nodes), r1 = ldg4(B.nodes + 1);
+                        float4 r0, r1;
+                        ldg8(B.nodes, r0, r1);
                         if (COUNT) cnt.blas_nodes++;
                         w0 = __float_as_uint(r0.w);
                         w1 = __float_as_uint(r1.w);
@@ -348,7 +354,9 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
                     uint2 e[4];
                     if constexpr (LAY == 1) {
                         const float4* qp = B.qnodes + 4ull * w0;
-                        const float4 q0 = ldg4(qp), q1 = ldg4(qp + 1), q2 = ldg4(qp + 2), q3 = ldg4(qp + 3);
+                        float4 q0, q1, q2, q3;
+                        ldg8(qp, q0, q1);
+                        ldg8(qp + 2, q2, q3);
                         if (COUNT) cnt.blas_nodes += 2;   // 64 bytes, as a binary child pair
                         const uint32_t meta = __float_as_uint(q0.w);
                         const float sx = __uint_as_float((meta & 0xFFu) << 23);
@@ -373,8 +381,11 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
                         }
                     } else {
                         const float4* wp = B.qnodes + 8ull * w0;
-                        const float4 xl = ldg4(wp), xh = ldg4(wp + 1), yl = ldg4(wp + 2), yh = ldg4(wp + 3);
-                        const float4 zl = ldg4(wp + 4), zh = ldg4(wp + 5), en = ldg4(wp + 6), cn = ldg4(wp + 7);
+                        float4 xl, xh, yl, yh, zl, zh, en, cn;
+                        ldg8(wp, xl, xh);
+                        ldg8(wp + 2, yl, yh);
+                        ldg8(wp + 4, zl, zh);
+                        ldg8(wp + 6, en, cn);
                         if (COUNT) cnt.blas_nodes += 4;   // 128 bytes, as two binary child pairs
                         const uint32_t nch = __float_as_uint(cn.x) >> 24;
                         auto lane4 = [](const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; };
@@ -419,7 +430,9 @@ __device__ __forceinline__ void trace_persistent(const SceneRefs& S, IO& io, uin
                                 : !in_bounds(w0 + 1ull, B.node_count, S.status)) {
                     pop = true;
                 } else {
-                    const float4 a0 = ldg4(pa), a1 = ldg4(pa + 1), b0 = ldg4(pa + 2), b1 = ldg4(pa + 3);
+                    float4 a0, a1, b0, b1;
+                    ldg8(pa, a0, a1);
+                    ldg8(pa + 2, b0, b1);
                     if (COUNT) { if (level == 0u) cnt.tlas_nodes += 2; else cnt.blas_nodes += 2; }
                     float dl, dr;
                     bool hl, hr;   // the children entered before the current hit
