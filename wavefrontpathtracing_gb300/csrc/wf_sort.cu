@@ -3,14 +3,15 @@
 // codes in the scene's bounding box, so the rays a GPU holds at once start
 // close together and read the same BVH nodes from L2 instead of each going to
 // DRAM.  The order comes from a stable LSD radix sort of (code, ray index)
-// pairs written here: three 8-bit passes of upsweep (digit counts per tile),
-// an exclusive scan of the counts (digit-major, so equal digits keep their
+// pairs written here: two 8-bit passes, over the codes' upper 16 bits, of
+// upsweep (digit counts per tile), an exclusive scan of the counts (digit-major, so equal digits keep their
 // tiles' order) and a downsweep that ranks each tile's keys in order (warp
 // match + per-warp counts) and scatters them.  Rays with equal codes keep
 // their input order; when every origin falls in one cell (camera rays) the key
 // pass says so in a device flag, the sort passes return at once and the rays
 // are traced in their own order.  The hits land at each ray's own index;
 // which ray a lane traces never changes a result.
+#include <algorithm>
 #include "wf_kernels.h"
 
 namespace wf {
@@ -39,28 +40,10 @@ __device__ __forceinline__ uint32_t cell8(float x, float lo, float inv) {
     return (uint32_t)(u * 256.0f) & 0xFFu;
 }
 
-// WF_SORT_DIR_BITS = k > 0: the key's top 24 - 3k bits are the origin's
-// Morton code at 8 - k bits per axis and its low 3k bits the Morton code of
-// the direction quantised to k bits per axis, so rays that start in one cell
-// are also ordered by where they go.
-#ifndef WF_SORT_DIR_BITS
-#define WF_SORT_DIR_BITS 0
-#endif
-static_assert(WF_SORT_DIR_BITS >= 0 && WF_SORT_DIR_BITS <= 4, "WF_SORT_DIR_BITS: 0..4");
-
 __device__ __forceinline__ uint32_t ray_key(const float4* __restrict__ rays, uint32_t i, float3 lo, float3 inv) {
     const float4 o = __ldg(rays + 2ull * i);
-    constexpr int k = WF_SORT_DIR_BITS;
-    uint32_t key = (spread8(cell8(o.x, lo.x, inv.x) >> k) << 2) | (spread8(cell8(o.y, lo.y, inv.y) >> k) << 1) |
-                   spread8(cell8(o.z, lo.z, inv.z) >> k);
-    if constexpr (k > 0) {
-        const float4 d = __ldg(rays + 2ull * i + 1);
-        // direction components in [-1, 1] -> [0, 1] -> k bits (cell8 clamps and maps NaN to 0)
-        const uint32_t dx = cell8(d.x, -1.0f, 0.5f) >> (8 - k), dy = cell8(d.y, -1.0f, 0.5f) >> (8 - k),
-                       dz = cell8(d.z, -1.0f, 0.5f) >> (8 - k);
-        key = (key << (3 * k)) | (spread8(dx) << 2) | (spread8(dy) << 1) | spread8(dz);
-    }
-    return key;
+    return (spread8(cell8(o.x, lo.x, inv.x)) << 2) | (spread8(cell8(o.y, lo.y, inv.y)) << 1) |
+           spread8(cell8(o.z, lo.z, inv.z));
 }
 
 // Key = 24-bit Morton code of the origin in the scene box (clamped), value =
@@ -279,11 +262,17 @@ cudaError_t launch_reorder_rays(const float4* rays, uint32_t n, const float4* ro
     unsigned long long* scattered = reinterpret_cast<unsigned long long*>(scratch + ((words - 2) & ~size_t(1)));
     cudaError_t e = cudaMemsetAsync(varied, 0, 4 * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
-    k_origin_keys<<<grid_for(n, 256), 256, 0, stream>>>(rays, n, root, has_scene, k0, v0, varied, scattered);
+    // eight blocks per SM walk the rays: each warp ends with atomics on one
+    // address, and a warp per 32 rays spent 190 of its 4.2M rays' us on those
+    k_origin_keys<<<std::min(grid_for(n, 256), 8u * (unsigned)sm_count()), 256, 0, stream>>>(rays, n, root, has_scene, k0, v0, varied, scattered);
     k_sort_decision<<<1, 1, 0, stream>>>(varied, scattered, n);
     e = cudaGetLastError();
-    for (int pass = 0; pass < 3 && e == cudaSuccess; ++pass) {
-        const int shift = 8 * pass;
+    // The 65,536 cells of the codes' upper 16 bits are fine enough, a third pass
+    // costs more than it gains: 4.2M rays against 2M / 1M / 20k triangles 4.34 /
+    // 4.43 / 2.19 ms with three, 4.29 / 4.39 / 2.12 with two (4.46 / 4.57 / 2.33
+    // with three and a warp per 32 rays above); 4 bits lower, 4.54.
+    for (int pass = 0; pass < 2 && e == cudaSuccess; ++pass) {
+        const int shift = 8 + 8 * pass;
         k_upsweep<<<tiles, kSortThreads, 0, stream>>>(k0, n, shift, tiles, hist, varied);
         e = exclusive_scan(hist, (uint64_t)kRadix * tiles, sums, varied, stream);
         if (e != cudaSuccess) break;
