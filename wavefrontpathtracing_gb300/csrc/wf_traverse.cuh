@@ -37,7 +37,8 @@
 // step per lane and iteration before) with the world ray's reciprocal kept
 // through an instance: 9.91 ms, 1.02, 316 us, 5.49 ms, and a whole-wave 256x256
 // frame 222 -> 172 us; then nodes and instance rows in 32-byte loads, half the
-// requests: 9.53 ms, 1.02, 298 us, 4.46 ms (quantized and exact 4-wide: 6.02 ->
+// requests: 9.53 ms, 1.02, 298 us, 4.46 ms, and with new rays at 12 idle lanes
+// again 9.29, 1.02, 290, 4.44 (quantized and exact 4-wide: 6.02 ->
 // 6.01, 7.04 -> 6.07).
 #pragma once
 #include <type_traits>
@@ -69,11 +70,12 @@ constexpr int kTraceBlock = WF_TRACE_BLOCK;
 #ifndef WF_TRACE_RING
 #define WF_TRACE_RING 8
 #endif
-// A warp takes new rays once this many of its lanes are idle (or all are); 8 /
-// 12 / 16: 4.2M incoherent closest-hit rays 5.69 / 5.58 / 5.54 ms, the others
-// within 0.5 % between 12 and 16.
+// A warp takes new rays once this many of its lanes are idle (or all are).  8 /
+// 10 / 12 / 14 / 16: 1080p instanced frame 9.34 / 9.30 / 9.29 / 9.34 / 9.52 ms, 1M
+// any-hit rays 290 / 289 / 290 / 293 / 298 us, a batch of scenes 8.69 / 8.60 /
+// 8.54 / 8.53 / 8.46 ms.
 #ifndef WF_TRACE_REFILL
-#define WF_TRACE_REFILL 16
+#define WF_TRACE_REFILL 12
 #endif
 constexpr int kRefill = WF_TRACE_REFILL;
 // Interior visits per loop iteration (binary layout), unrolled.  Each costs the
