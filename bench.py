@@ -797,9 +797,13 @@ def run_ours(args, rank, world, local):
                            "trace_schedule": ("fused" if args.fused_connect else
                                               f"separate, shadow rays fused from depth {args.fused_from_depth}"
                                               if args.fused_from_depth else "separate"),
+                           # the reference's primary ray has no jitter: a pixel's samples share it
+                           "camera_rays": "traced once per pixel and wave, counted once per path",
                            "l2": "256 MiB buffer written between timed frames; working set > L2"},
                 "spp_per_s": round(spp_per_s, 3),
                 "rays_per_step": rays // args.steps,
+                # without the camera rays that share another path's (one wave holds a frame's samples)
+                "rays_traced_per_step": rays // args.steps - (c["paths"] - W * H),
                 "gpu_launches": launches,
                 "stages_ms": {k: round(last[f"ms_{k}"], 3) for k in ("generate", "extend", "shade", "connect", "post",
                                                                         "tail")},

@@ -23,9 +23,9 @@
 // new rays in groups through one atomic per warp (kRefill idle lanes, or all
 // of them) from a per-launch counter.
 //
-// What bounds it: issue slots (61-74 % busy, most of it integer, compare and
+// What bounds it: issue slots (50-60 % busy, most of it integer, compare and
 // min / max work around the box tests) and the latency of the dependent node
-// loads at 12-14 active lanes of 32.  So the loop carries as little as it can:
+// loads at 13-15 active lanes of 32.  So the loop carries as little as it can:
 // TLAS nodes are read as child pairs in the BLAS's form, which makes an interior
 // step one code path with one pointer for both levels and a leaf test one
 // compare, and one ballot per iteration serves hand-out and termination
