@@ -832,8 +832,8 @@ def run_ours(args, rank, world, local):
                              "achieved": round(achieved, 1),
                              "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                              "frac": round(achieved / peak, 4), "traffic": traffic, "traffic_source": traffic_src,
-                             # depth 0 carries 82 % of the rays: 16 identical camera rays per pixel share a
-                             # warp, so one fetch serves 16 of them; the secondary depths are the real traversal
+                             # depth 0 carries 74 % of the counted rays: the 16 camera rays of a pixel are one
+                             # traced ray, whose fetches count 16 times; the secondary depths are the real traversal
                              "per_depth": per_depth, "frac_secondary": secondary["frac"] if secondary else None,
                              "secondary": secondary, "connect": connect, "solo": solo,
                              "alg_bytes_per_launch": int(bytes_per_launch),
