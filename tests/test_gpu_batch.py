@@ -171,3 +171,17 @@ def test_batch_call_order_and_argument_errors(batch_case):
             b.read_image(0)
         assert e.value.status == -7                      # nothing rendered
         b.close()
+
+
+@pytest.mark.parametrize("capacity,threshold", [(1031, 1.0), (1777, 0.3), (1 << 15, 0.9)])
+def test_split_pixels_share_the_right_camera_ray(batch_case, capacity, threshold):
+    """Admissions that end inside a pixel's samples: the rest of the pixel is
+    admitted later, behind continuing paths, and traces its camera ray again."""
+    meshes, descs, want = batch_case
+    with Renderer(8, 8) as r:
+        b = make_batch(r, meshes, descs)
+        b.set_config(capacity=capacity, regen_threshold=threshold, block=128)
+        b.render(frame_seed=SEED, **RENDER)
+        for k in range(len(descs)):
+            assert_same(b.read_image(k), want[k], f"scene {k}")
+        b.close()

@@ -22,8 +22,10 @@
 // parity); the next shade waits for it.
 //
 // Camera paths are numbered scene by scene, pixel-major inside a scene
-// (path = path_base + pixel * spp + sample, so a pixel's identical camera rays
-// share a warp), and admitted in that order.  A
+// (path = path_base + pixel * spp + sample), and admitted in that order.  A
+// pixel's camera rays are identical, so of those admitted together only the
+// first is traced and the others shade its hit (11 scenes of 1 to 16 samples: 8.53
+// -> 8.13 ms; in lockstep in one warp they cost it one ray's steps before).  A
 // path's random numbers are keyed by (scene-local pixel, sample, depth) as in
 // wf_render, its radiance is summed in the same order, and each finished path
 // stores its radiance at its own index; the resolve adds a pixel's samples in
@@ -77,6 +79,7 @@ struct BatchQueues {
     float4* qL[2];
     float4* h_tuvp;
     uint32_t* h_inst;
+    uint32_t* lead;   // pool entries of the admitted camera rays to trace, one per pixel
     float4* s_o[2];   // by iteration parity: {origin, tmax}
     float4* s_d[2];   // {direction, target}: pool slot of the continuing path, or kFinishedBit | camera path
     float4* s_c[2];   // {contribution, scene}
@@ -91,6 +94,7 @@ struct BatchCtl {
     uint32_t shadow[2];       // shadow rays of the iteration on queue k
     uint32_t fetch[3];        // persistent traversal hand-out counters: extend, connect on queue 0 / 1
     uint32_t regen_n, regen_g0, regen_slot0;
+    uint32_t trace_n;         // extension rays: the continuing paths, then the admitted paths' shared camera rays
     uint32_t next, total;     // next camera path to admit, number of camera paths
     uint32_t capacity, threshold;
     uint32_t iter, stall, stall_limit, done, body_runs;
@@ -118,6 +122,7 @@ __global__ void k_bbegin(BatchCtl* c, int cur) {
     c->regen_n = take;
     c->regen_g0 = c->next;
     c->regen_slot0 = n;
+    c->trace_n = n;   // k_bregen adds its camera rays
     c->next += take;
     c->count[cur ^ 1] = 0;
     c->shadow[cur] = 0;
@@ -130,8 +135,13 @@ __global__ void k_bbegin(BatchCtl* c, int cur) {
 // path-state reset is the entry's initial throughput / radiance).
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_bregen(const BatchScene* sc, const uint32_t* pbase, uint32_t ns,
-                                                  BatchQueues Q, const BatchCtl* c, int cur) {
+                                                  BatchQueues Q, BatchCtl* c, int cur) {
     const uint32_t m = c->regen_n, g0 = c->regen_g0, s0 = c->regen_slot0;
+    if (m == 0u || !in_bounds(g0, Q.total_paths, Q.status)) return;
+    // pixels are numbered over the scenes as their paths are, so a pixel's place
+    // among the admitted ones follows from its number
+    const BatchScene& S0 = sc[scene_of(pbase, ns, g0)];
+    const uint32_t pix0 = S0.pix_base + (g0 - S0.path_base) / S0.spp;
     // queue pointers picked by selects: a dynamic index into the parameter
     // arrays would copy them to local memory
     float4* const qo = cur ? Q.qo[1] : Q.qo[0];
@@ -148,6 +158,9 @@ __global__ void __launch_bounds__(BLOCK) k_bregen(const BatchScene* sc, const ui
         V3 o, d;
         primary_ray(S, pixel % S.width, pixel / S.width, o, d);
         const uint32_t slot = s0 + j;
+        const uint32_t nth = S.pix_base + pixel - pix0;
+        if ((sample == 0u || j == 0u) && in_bounds(nth, Q.capacity, Q.status)) Q.lead[nth] = slot;
+        if (j == m - 1u) c->trace_n = s0 + nth + 1u;
         qo[slot] = make_float4(o.x, o.y, o.z, __uint_as_float(kFlagSpecular | (s << kSceneShift)));
         qd[slot] = make_float4(d.x, d.y, d.z, __uint_as_float(pixel));
         qT[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
@@ -155,7 +168,11 @@ __global__ void __launch_bounds__(BLOCK) k_bregen(const BatchScene* sc, const ui
     }
 }
 
+// The rays of the extension launch: entry k of the queue below the admitted
+// paths, then the admitted pixels' shared camera rays.
 struct BatchExtendIO {
+    const uint32_t* lead;
+    const BatchCtl* c;
     const float4* qo;
     const float4* qd;
     float4* tuvp;
@@ -163,16 +180,22 @@ struct BatchExtendIO {
     const uint32_t* roots;
     uint32_t nscenes;    // checked builds
     uint32_t* status;
-    __device__ __forceinline__ void load(uint32_t i, V3& o, V3& d, float& tmax, bool& nc) const {
+    __device__ __forceinline__ uint32_t entry(uint32_t k) const {
+        const uint32_t s0 = c->regen_slot0;
+        return k < s0 ? k : lead[k - s0];
+    }
+    __device__ __forceinline__ void load(uint32_t k, V3& o, V3& d, float& tmax, bool& nc) const {
+        const uint32_t i = entry(k);
         const float4 a = qo[i], b = qd[i];
         o = xyz(a); d = xyz(b); tmax = FLT_MAX;
         nc = (__float_as_uint(a.w) & kFlagInside) != 0u;
     }
-    __device__ __forceinline__ uint32_t root(uint32_t i, const SceneRefs&) const {
-        const uint32_t scene = __float_as_uint(qo[i].w) >> kSceneShift;
+    __device__ __forceinline__ uint32_t root(uint32_t k, const SceneRefs&) const {
+        const uint32_t scene = __float_as_uint(qo[entry(k)].w) >> kSceneShift;
         return in_bounds(scene, nscenes, status) ? roots[scene] : kInvalid;
     }
-    __device__ __forceinline__ void store(uint32_t i, const Hit& h, bool) const {
+    __device__ __forceinline__ void store(uint32_t k, const Hit& h, bool) const {
+        const uint32_t i = entry(k);
         tuvp[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
         inst[i] = h.inst;
     }
@@ -264,13 +287,16 @@ __global__ void __launch_bounds__(BLOCK) k_bshade(ShadeRefs SH, const BatchScene
             K.env_tex = S.env_tex; K.view_mode = 0u; K.far_plane = 1.0f;
             ShadeIn in;
             in.rd = xyz(b);
-            in.tuvp = Q.h_tuvp[i];
-            in.inst = Q.h_inst[i];
+            in.sample = __float_as_uint(L4.w);
+            // a camera path's hit is its pixel's first admitted one's
+            const uint32_t first = c->regen_slot0;
+            const uint32_t hit = depth ? i : i - min(in.sample, i - first);
+            in.tuvp = Q.h_tuvp[hit];
+            in.inst = Q.h_inst[hit];
             in.T = xyz(T4);
             in.last_pdf = T4.w;
             in.flags = f & 0xFFu;
             in.pixel = pixel;
-            in.sample = __float_as_uint(L4.w);
             in.depth = depth;
             shade_one(SH, K, in, none, 0u, 0u, o);
             if (o.has_add) {
@@ -432,7 +458,7 @@ struct wf_batch {
     uint32_t pool_block = 0;
     DBuf<float4> q[8];
     DBuf<float4> h_tuvp, s_o[2], s_d[2], s_c[2];
-    DBuf<uint32_t> h_inst;
+    DBuf<uint32_t> h_inst, lead;
     BatchCtl* ctl = nullptr;
     BatchCtl* ctl_host = nullptr;   // pinned
 
@@ -584,7 +610,7 @@ int ensure_pool(wf_batch* b) {
     int rc;
     for (int k = 0; k < 8; ++k)
         if ((rc = b->q[k].reserve(C))) return rc;
-    if ((rc = b->h_tuvp.reserve(C)) || (rc = b->h_inst.reserve(C))) return rc;
+    if ((rc = b->h_tuvp.reserve(C)) || (rc = b->h_inst.reserve(C)) || (rc = b->lead.reserve(C))) return rc;
     for (int k = 0; k < 2; ++k)
         if ((rc = b->s_o[k].reserve(C)) || (rc = b->s_d[k].reserve(C)) || (rc = b->s_c[k].reserve(C))) return rc;
     if (!b->ctl) {
@@ -613,6 +639,7 @@ BatchQueues queues(wf_batch* b) {
     }
     Q.h_tuvp = b->h_tuvp.p;
     Q.h_inst = b->h_inst.p;
+    Q.lead = b->lead.p;
     for (int k = 0; k < 2; ++k) {
         Q.s_o[k] = b->s_o[k].p;
         Q.s_d[k] = b->s_d[k].p;
@@ -684,10 +711,11 @@ int enqueue_iteration(wf_batch* b, int k, bool join_prev, bool join_self, cudaGr
     BCUDA(cudaGetLastError());
     BCUDA(regen_or_shade(false, b, SH, Q, cur, st));
     BatchExtendIO ex;
+    ex.lead = Q.lead; ex.c = b->ctl;
     ex.qo = Q.qo[cur]; ex.qd = Q.qd[cur]; ex.tuvp = Q.h_tuvp; ex.inst = Q.h_inst; ex.roots = b->d_roots.p;
     ex.nscenes = b->nscenes; ex.status = status;
     auto ke = k_btrace<false, BatchExtendIO>;
-    ke<<<persistent_grid(ke), kTraceBlock, 0, st>>>(S, ex, &b->ctl->count[cur], &b->ctl->fetch[0], status);
+    ke<<<persistent_grid(ke), kTraceBlock, 0, st>>>(S, ex, &b->ctl->trace_n, &b->ctl->fetch[0], status);
     BCUDA(cudaGetLastError());
     const int kp = (k + kBodyIterations - 1) % kBodyIterations;
     if (join_prev) BCUDA(cudaStreamWaitEvent(st, b->ev_conn[kp], 0));   // both add to the path radiance
@@ -900,7 +928,7 @@ int wf_batch_destroy(wf_batch* b) {
     b->lights.release(); b->blas.release(); b->stri.release(); b->d_scenes.release();
     b->out_L.release(); b->image.release();
     for (auto& q : b->q) q.release();
-    b->h_tuvp.release(); b->h_inst.release();
+    b->h_tuvp.release(); b->h_inst.release(); b->lead.release();
     for (int k = 0; k < 2; ++k) { b->s_o[k].release(); b->s_d[k].release(); b->s_c[k].release(); }
     for (int k = 0; k < kBodyIterations; ++k) {
         if (b->ev_shade[k]) cudaEventDestroy(b->ev_shade[k]);
