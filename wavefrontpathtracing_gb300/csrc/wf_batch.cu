@@ -355,13 +355,7 @@ __global__ void k_bresolve(const BatchScene* sc, const uint32_t* pixbase, uint32
         const BatchScene& S = sc[s];
         const uint32_t p = q - S.pix_base;
         float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (uint32_t k = 0; k < S.spp; ++k) {
-            const float4 L = out_L[(size_t)S.path_base + (size_t)p * S.spp + k];
-            acc.x = acc.x + L.x;
-            acc.y = acc.y + L.y;
-            acc.z = acc.z + L.z;
-            acc.w = acc.w + 1.0f;
-        }
+        sum_samples(out_L + (size_t)S.path_base + (size_t)p * S.spp, S.spp, acc);
         image[q] = acc.w > 0.0f ? make_float4(acc.x / acc.w, acc.y / acc.w, acc.z / acc.w, acc.w)
                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }

@@ -245,13 +245,7 @@ __global__ void k_wave_resolve(RenderBuffers B, WaveParams W) {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < W.np; p += stride) {
         float4 acc = B.accum[W.pix0 + p];
-        for (uint32_t s = 0; s < W.nsamples; ++s) {
-            const float4 L = B.ps_L[(size_t)p * W.nsamples + s];
-            acc.x = acc.x + L.x;
-            acc.y = acc.y + L.y;
-            acc.z = acc.z + L.z;
-            acc.w = acc.w + 1.0f;
-        }
+        sum_samples(B.ps_L + (size_t)p * W.nsamples, W.nsamples, acc);
         B.accum[W.pix0 + p] = acc;
     }
 }
