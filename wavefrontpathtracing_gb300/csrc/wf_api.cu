@@ -146,7 +146,7 @@ struct wf_ctx {
     DevBuf<float4> tri_albedo;              // per scene triangle (wf_scene_set_albedo)
     DevBuf<uint32_t> inst_tri_offset;
     DevBuf<float4> dimage, g_albedo;        // adjoint buffers
-    DevBuf<float> g_em_rep;                 // adjoint: emitter gradients, 32 replicas
+    DevBuf<double> g_em_rep;                // adjoint: emitter gradients, 32 replicas
     DevBuf<float4> L_comp;                  // adjoint: rounding errors of the path radiance sums
     DevBuf<uint8_t> tape;                   // adjoint: the forward pass's hits and visibilities
 
@@ -1727,7 +1727,7 @@ int wf_adjoint(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
     if ((rc = begin_call(c, false))) return rc;
     WF_CUDA(h2d(c, c->dimage.p, dimg.data(), dimg.size() * sizeof(float4)));
     WF_CUDA(cudaMemsetAsync(c->g_albedo.p, 0, (uint64_t)replicas * ntri * sizeof(float4), c->stream));
-    WF_CUDA(cudaMemsetAsync(c->g_em_rep.p, 0, 32ull * std::max<uint64_t>(ninst, 1) * sizeof(float), c->stream));
+    WF_CUDA(cudaMemsetAsync(c->g_em_rep.p, 0, 32ull * std::max<uint64_t>(ninst, 1) * sizeof(double), c->stream));
     Pass P = make_pass(c, s, o, frame_seed);
     P.fused = false;   // the shadow rays' launches record what they find
     P.fuse_from = 0;
@@ -1762,10 +1762,10 @@ int wf_adjoint(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
     WF_CUDA(launch_reduce_replicas(c->g_albedo.p, (uint32_t)ntri, replicas, c->stream));
     c->launches++;
     std::vector<float4> ga(ntri);
-    std::vector<float> gr(32ull * ninst);
+    std::vector<double> gr(32ull * ninst);
     WF_CUDA(d2h(c, ga.data(), c->g_albedo.p, ntri * sizeof(float4)));
     if (ninst) {
-        WF_CUDA(d2h(c, gr.data(), c->g_em_rep.p, gr.size() * sizeof(float)));
+        WF_CUDA(d2h(c, gr.data(), c->g_em_rep.p, gr.size() * sizeof(double)));
     }
     if ((rc = end_call(c))) return rc;
     WF_CUDA(cudaStreamSynchronize(c->stream));
@@ -1776,7 +1776,7 @@ int wf_adjoint(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
     }
     for (uint64_t i = 0; i < ninst; ++i) {
         double e = 0.0;
-        for (uint32_t r = 0; r < 32; ++r) e = e + (double)gr[(size_t)r * ninst + i];
+        for (uint32_t r = 0; r < 32; ++r) e = e + gr[(size_t)r * ninst + i];
         d_emission[i] = (float)e;
     }
     c->stats.paths = (uint64_t)npix * o->spp;

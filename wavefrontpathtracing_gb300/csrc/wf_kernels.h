@@ -39,7 +39,7 @@ struct AdjointRefs {
     uint32_t replicas;            // power of two; a warp adds into replica (block ^ warp) % replicas
     uint32_t triangles;
     const float4* L_final_lo;     // per path: the forward pass's ps_Lc (L_final + L_final_lo = the exact sum)
-    float* g_em_rep;              // emitter gradients: 32 replicas x instances
+    double* g_em_rep;             // emitter gradients: 32 replicas x instances (doubles: see k_replay)
     uint32_t instances;
 };
 

@@ -513,7 +513,7 @@ __device__ __forceinline__ void shade_one(const ShadeRefs& SH, const ShadeCtl& K
 }
 
 // Warp-aggregated atomic add of v to g[key] (one atomic per distinct key in the warp).
-__device__ __forceinline__ void warp_add_by_key(float* g, uint32_t key, float v) {
+__device__ __forceinline__ void warp_add_by_key(double* g, uint32_t key, double v) {
     bool pending = key != kInvalid;
     for (;;) {
         const unsigned rem = __ballot_sync(0xffffffffu, pending);
@@ -521,7 +521,7 @@ __device__ __forceinline__ void warp_add_by_key(float* g, uint32_t key, float v)
         const int leader = __ffs(rem) - 1;
         const uint32_t k = __shfl_sync(0xffffffffu, key, leader);
         const bool mine = pending && key == k;
-        float s = mine ? v : 0.0f;
+        double s = mine ? v : 0.0;
         for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
         if ((int)(threadIdx.x & 31) == leader) atomicAdd(&g[k], s);
         if (mine) pending = false;
