@@ -113,6 +113,8 @@ cudaError_t launch_trace_aos(const SceneRefs& S, const void* rays, uint32_t n, v
 // to a device word that stays 0 when every origin fell in one cell (the sort
 // then did nothing and perm must not be used).
 size_t reorder_scratch_words(uint32_t n);
+// Its kernels: keys, the decision, then upsweep + 3 scan kernels + downsweep per pass.
+constexpr int kReorderPasses = 2, kReorderLaunches = 2 + 5 * kReorderPasses;
 cudaError_t launch_reorder_rays(const float4* rays, uint32_t n, const float4* root, bool has_scene,
                                 uint32_t* scratch, const uint32_t** perm, const uint32_t** varied,
                                 cudaStream_t stream);

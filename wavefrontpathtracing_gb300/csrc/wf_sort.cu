@@ -273,7 +273,7 @@ cudaError_t launch_reorder_rays(const float4* rays, uint32_t n, const float4* ro
     // costs more than it gains: 4.2M rays against 2M / 1M / 20k triangles 4.34 /
     // 4.43 / 2.19 ms with three, 4.29 / 4.39 / 2.12 with two (4.46 / 4.57 / 2.33
     // with three and a warp per 32 rays above); 4 bits lower, 4.54.
-    for (int pass = 0; pass < 2 && e == cudaSuccess; ++pass) {
+    for (int pass = 0; pass < kReorderPasses && e == cudaSuccess; ++pass) {
         const int shift = 8 + 8 * pass;
         k_upsweep<<<tiles, kSortThreads, 0, stream>>>(k0, n, shift, tiles, hist, varied);
         e = exclusive_scan(hist, (uint64_t)kRadix * tiles, sums, varied, stream);
