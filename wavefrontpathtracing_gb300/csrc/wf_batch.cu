@@ -708,8 +708,8 @@ int enqueue_iteration(wf_batch* b, int k, bool join_prev, bool join_self, cudaGr
     ex.lead = Q.lead; ex.c = b->ctl;
     ex.qo = Q.qo[cur]; ex.qd = Q.qd[cur]; ex.tuvp = Q.h_tuvp; ex.inst = Q.h_inst; ex.roots = b->d_roots.p;
     ex.nscenes = b->nscenes; ex.status = status;
-    auto ke = k_btrace<false, BatchExtendIO>;
-    ke<<<persistent_grid(ke), kTraceBlock, 0, st>>>(S, ex, &b->ctl->trace_n, &b->ctl->fetch[0], status);
+    constexpr auto ke = k_btrace<false, BatchExtendIO>;
+    ke<<<persistent_grid<ke, kTraceBlock>(), kTraceBlock, 0, st>>>(S, ex, &b->ctl->trace_n, &b->ctl->fetch[0], status);
     BCUDA(cudaGetLastError());
     const int kp = (k + kBodyIterations - 1) % kBodyIterations;
     if (join_prev) BCUDA(cudaStreamWaitEvent(st, b->ev_conn[kp], 0));   // both add to the path radiance
@@ -720,8 +720,8 @@ int enqueue_iteration(wf_batch* b, int k, bool join_prev, bool join_self, cudaGr
     cn.so = Q.s_o[cur]; cn.sd = Q.s_d[cur]; cn.sc = Q.s_c[cur]; cn.roots = b->d_roots.p; cn.qL = Q.qL[cur ^ 1];
     cn.nscenes = b->nscenes; cn.capacity = b->cfg.capacity; cn.total_paths = b->total_paths; cn.status = status;
     cn.out_L = Q.out_L;
-    auto kc = k_btrace<true, BatchConnectIO>;
-    kc<<<persistent_grid(kc), kTraceBlock, 0, b->side>>>(S, cn, &b->ctl->shadow[cur], &b->ctl->fetch[1 + cur], status);
+    constexpr auto kc = k_btrace<true, BatchConnectIO>;
+    kc<<<persistent_grid<kc, kTraceBlock>(), kTraceBlock, 0, b->side>>>(S, cn, &b->ctl->shadow[cur], &b->ctl->fetch[1 + cur], status);
     BCUDA(cudaGetLastError());
     BCUDA(cudaEventRecord(b->ev_conn[k], b->side));
     if (join_self) BCUDA(cudaStreamWaitEvent(st, b->ev_conn[k], 0));
@@ -736,8 +736,8 @@ int build_graph(wf_batch* b) {
     drop_graph(b);
     cudaStream_t st = ctx_stream(b->ctx);
     // occupancy queries before capture
-    (void)persistent_grid(k_btrace<false, BatchExtendIO>);
-    (void)persistent_grid(k_btrace<true, BatchConnectIO>);
+    (void)persistent_grid<k_btrace<false, BatchExtendIO>, kTraceBlock>();
+    (void)persistent_grid<k_btrace<true, BatchConnectIO>, kTraceBlock>();
     (void)sm_count();
     BCUDA(cudaGraphCreate(&b->graph, 0));
     cudaGraphConditionalHandle h;

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kTraceBlock, WF_FINISH_MIN_BLOCKS)
 
 cudaError_t launch_finish(const SceneRefs& S, const ShadeRefs& SH, const RenderBuffers& B, const WaveParams& W,
                           uint32_t depth, unsigned long long* totals, cudaStream_t stream) {
-    k_finish<<<persistent_grid(k_finish), kTraceBlock, 0, stream>>>(S, SH, B, W, depth,
+    k_finish<<<persistent_grid<k_finish, kTraceBlock>(), kTraceBlock, 0, stream>>>(S, SH, B, W, depth,
                                                                     B.counts + 2 * kMaxDepth + depth, totals);
     return cudaGetLastError();
 }

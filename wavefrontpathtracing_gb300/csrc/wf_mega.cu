@@ -114,23 +114,13 @@ __global__ void __launch_bounds__(kMegaBlock) k_mega(SceneRefs S, ShadeRefs SH, 
     finish(overflow, B.status, n_ext, n_con, totals);
 }
 
-template <class K>
-unsigned mega_grid(K kernel) {
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMegaBlock, 0);
-        if (per_sm <= 0) per_sm = 1;
-    }
-    return (unsigned)(sm_count() * per_sm);
-}
-
 }  // namespace
 
 cudaError_t launch_megakernel(const SceneRefs& S, const ShadeRefs& SH, const RenderBuffers& B, const WaveParams& W,
                               uint32_t* fetch, unsigned long long* totals, cudaStream_t stream) {
     cudaError_t e = cudaMemsetAsync(fetch, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
-    k_mega<<<mega_grid(k_mega), kMegaBlock, 0, stream>>>(S, SH, B, W, fetch, totals);
+    k_mega<<<persistent_grid<k_mega, kMegaBlock>(), kMegaBlock, 0, stream>>>(S, SH, B, W, fetch, totals);
     return cudaGetLastError();
 }
 

@@ -1,6 +1,8 @@
 // wf_trace.cu — ray-query kernels: extend (closest hit, extend.hlsl:25-40),
 // connect (any-hit shadow rays; the reference's connect.hlsl is empty) and the
 // stand-alone query behind wf_trace.
+#include <atomic>
+
 #include "wf_shade.cuh"
 #include "wf_traverse.cuh"
 
@@ -141,8 +143,8 @@ __global__ void __launch_bounds__(kTraceBlock, LAY ? WF_TRACE_QB_MIN_BLOCKS : WF
 template <bool ANY, bool COUNT, int LAY, class IO>
 void launch_layout(const SceneRefs& S, const IO& io, const uint32_t* count_ptr, uint32_t count, uint32_t* fetch,
                    uint32_t* status, Counters* counters, unsigned long long* total, cudaStream_t stream) {
-    auto k = k_trace<ANY, COUNT, LAY, IO>;
-    k<<<persistent_grid(k), kTraceBlock, 0, stream>>>(S, io, count_ptr, count, fetch, status, counters, total);
+    constexpr auto k = k_trace<ANY, COUNT, LAY, IO>;
+    k<<<persistent_grid<k, kTraceBlock>(), kTraceBlock, 0, stream>>>(S, io, count_ptr, count, fetch, status, counters, total);
 }
 template <bool ANY, bool COUNT, class IO>
 cudaError_t launch(const SceneRefs& S, const IO& io, const uint32_t* count_ptr, uint32_t count, uint32_t* fetch,
@@ -160,12 +162,12 @@ cudaError_t launch(const SceneRefs& S, const IO& io, const uint32_t* count_ptr, 
 
 int sm_count() {
     // per device (a process may drive different GPUs), queried once each
-    static int s_sms[64] = {};
+    static std::atomic<int> s_sms[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    int* slot = (dev >= 0 && dev < 64) ? &s_sms[dev] : nullptr;
-    if (slot && *slot > 0) return *slot;
-    int sms = 0;
+    std::atomic<int>* slot = (dev >= 0 && dev < 64) ? &s_sms[dev] : nullptr;
+    int sms = slot ? slot->load() : 0;
+    if (sms > 0) return sms;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (sms <= 0) sms = 1;
     if (slot) *slot = sms;
@@ -246,13 +248,13 @@ cudaError_t launch_trace_pair(const SceneRefs& S, const RenderBuffers& B, uint32
     const uint32_t* ns = B.counts + kMaxDepth + depth - 1;
     const uint32_t* ne = B.counts + depth;
     if (S.qbvh == 2u)
-        k_trace_pair<2><<<persistent_grid(k_trace_pair<2>), kTraceBlock, 0, stream>>>(S, io, ns, ne, fetch, B.status,
+        k_trace_pair<2><<<persistent_grid<k_trace_pair<2>, kTraceBlock>(), kTraceBlock, 0, stream>>>(S, io, ns, ne, fetch, B.status,
                                                                                        totals);
     else if (S.qbvh == 1u)
-        k_trace_pair<1><<<persistent_grid(k_trace_pair<1>), kTraceBlock, 0, stream>>>(S, io, ns, ne, fetch, B.status,
+        k_trace_pair<1><<<persistent_grid<k_trace_pair<1>, kTraceBlock>(), kTraceBlock, 0, stream>>>(S, io, ns, ne, fetch, B.status,
                                                                                        totals);
     else
-        k_trace_pair<0><<<persistent_grid(k_trace_pair<0>), kTraceBlock, 0, stream>>>(S, io, ns, ne, fetch, B.status,
+        k_trace_pair<0><<<persistent_grid<k_trace_pair<0>, kTraceBlock>(), kTraceBlock, 0, stream>>>(S, io, ns, ne, fetch, B.status,
                                                                                        totals);
     return cudaGetLastError();
 }

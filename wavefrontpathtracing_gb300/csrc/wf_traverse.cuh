@@ -43,6 +43,7 @@
 #pragma once
 #include <type_traits>
 #include "wf_device.cuh"
+#include "wf_grid.h"
 
 namespace wf {
 
@@ -681,8 +682,6 @@ __device__ __forceinline__ void flush_counters(const LocalCounters& c, Counters*
 #ifndef WF_TRACE_QB_MIN_BLOCKS
 #define WF_TRACE_QB_MIN_BLOCKS 8
 #endif
-int sm_count();
-
 // The traversal kernel: a persistent grid over count rays (read from
 // count_ptr on the device when it is non-null), rays handed out from *fetch.
 // total (optional) accumulates the number of rays of each launch.
@@ -697,17 +696,6 @@ __global__ void __launch_bounds__(kTraceBlock, LAY ? WF_TRACE_QB_MIN_BLOCKS : WF
     trace_persistent<ANY, COUNT, LAY>(S, io, n, fetch, c, overflow);
     if (overflow) atomicOr(status, ERRF_STACK);
     if (COUNT) flush_counters(c, counters);
-}
-
-// Resident blocks per SM for a kernel, queried once per instantiation.
-template <class K>
-inline unsigned persistent_grid(K kernel) {
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTraceBlock, 0);
-        if (per_sm <= 0) per_sm = 1;
-    }
-    return (unsigned)(sm_count() * per_sm);
 }
 
 }  // namespace wf
