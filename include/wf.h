@@ -234,7 +234,12 @@ int wf_abi_version(void);
 int wf_checked_build(void);
 /* Process-wide cap on the device memory the library allocates (all contexts
  * and batches); an allocation past it fails with WF_ERR_OOM and leaves the
- * caller's objects usable.  0 = no cap (the default). */
+ * caller's objects usable.  0 = no cap (the default).
+ * The library keeps idle blocks for its next calls: up to 256 MiB of scratch
+ * in the process (BLAS builds), and in each context the hits that its last
+ * wf_adjoint recorded (up to 4 GiB).  They do not count as used.  Any of the
+ * library's allocations that needs their room frees them; so do a limit that
+ * they exceed, and wf_destroy: of its context's own, of the last context all. */
 int wf_set_device_memory_limit(uint64_t bytes);
 int wf_get_device_memory_usage(uint64_t* out_bytes);
 /* The context's cudaStream_t, for callers that time or order work around it. */

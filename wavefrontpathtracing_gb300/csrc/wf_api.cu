@@ -148,7 +148,6 @@ struct wf_ctx {
     DevBuf<float4> dimage, g_albedo;        // adjoint buffers
     DevBuf<double> g_em_rep;                // adjoint: emitter gradients, 32 replicas
     DevBuf<float4> L_comp;                  // adjoint: rounding errors of the path radiance sums
-    DevBuf<uint8_t> tape;                   // adjoint: the forward pass's hits and visibilities
 
     // wavefront buffers
     bool buffers_ready = false;
@@ -624,25 +623,38 @@ std::unordered_map<void*, size_t> g_mem_blocks;
 uint64_t g_mem_used = 0, g_mem_limit = 0;   // limit 0: none
 
 // Scratch blocks kept between calls (cudaMalloc + cudaFree of a build's scratch
-// take 75 us for a few MB and 130 us for 130 MB, and cudaFree waits for the
-// whole device).  A kept block is idle: its last user's stream was synchronized
-// before it came back.  At most kKeptBytes are kept; all go back to the driver
+// take 75 us for a few MB and 130 us for 130 MB, of an adjoint's 587 MB 525, and
+// cudaFree waits for the whole device).  A kept block is idle: its last user's
+// stream was synchronized before it came back.  At most kKeptBytes are kept for
+// any call, and per context the last adjoint's hits; all go back to the driver
 // when an allocation fails, when the memory limit leaves no room for them and
-// when the last context is destroyed.  Idle blocks do not count as used.
+// when the last context is destroyed (a context's own with it).  Idle blocks do
+// not count as used.
 struct Kept {
     void* p;
     size_t bytes;
     int device;
+    const void* owner;
 };
 constexpr uint64_t kKeptBytes = 256ull << 20;
 std::vector<Kept> g_kept;
-uint64_t g_kept_bytes = 0;
+uint64_t g_kept_bytes = 0, g_kept_shared = 0;   // all; those without an owner
 uint32_t g_contexts = 0;
 
-void drop_kept() {   // g_mem_mutex held
-    for (const Kept& k : g_kept) cudaFree(k.p);
-    g_kept.clear();
-    g_kept_bytes = 0;
+// All with g_mem_mutex held.
+Kept take_kept(size_t i) {
+    const Kept k = g_kept[i];
+    g_kept.erase(g_kept.begin() + (long)i);
+    g_kept_bytes -= k.bytes;
+    if (!k.owner) g_kept_shared -= k.bytes;
+    return k;
+}
+void drop_kept() {
+    while (!g_kept.empty()) cudaFree(take_kept(g_kept.size() - 1).p);
+}
+void drop_owned(const void* owner) {
+    for (size_t i = g_kept.size(); i-- > 0;)
+        if (g_kept[i].owner == owner) cudaFree(take_kept(i).p);
 }
 }  // namespace
 
@@ -653,29 +665,31 @@ static void count_context(int by) {
     if (g_contexts == 0) drop_kept();
 }
 
-cudaError_t scratch_take(void** p, size_t bytes) {
+cudaError_t scratch_take(void** p, size_t bytes, const void* owner) {
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) {
         std::lock_guard<std::mutex> lock(g_mem_mutex);
+        auto fits = [&](const Kept& k) {
+            return k.device == dev && k.owner == owner && k.bytes >= bytes &&
+                   !(g_mem_limit && g_mem_used + k.bytes > g_mem_limit);
+        };
         size_t best = g_kept.size();
         for (size_t i = 0; i < g_kept.size(); ++i)
-            if (g_kept[i].device == dev && g_kept[i].bytes >= bytes &&
-                (best == g_kept.size() || g_kept[i].bytes < g_kept[best].bytes))
-                best = i;
-        if (best < g_kept.size() && !(g_mem_limit && g_mem_used + g_kept[best].bytes > g_mem_limit)) {
-            const Kept k = g_kept[best];
-            g_kept.erase(g_kept.begin() + (long)best);
-            g_kept_bytes -= k.bytes;
+            if (fits(g_kept[i]) && (best == g_kept.size() || g_kept[i].bytes < g_kept[best].bytes)) best = i;
+        if (best < g_kept.size()) {
+            const Kept k = take_kept(best);
             g_mem_blocks[k.p] = k.bytes;
             g_mem_used += k.bytes;
             *p = k.p;
             return cudaSuccess;
         }
     }
-    return dmalloc(p, bytes);
+    const cudaError_t e = dmalloc(p, bytes);
+    if (owner && e == cudaSuccess) scratch_drop(owner);   // the new one takes its place
+    return e;
 }
 
-void scratch_give(void* p) {
+void scratch_give(void* p, const void* owner) {
     if (!p) return;
     int dev = 0;
     const bool have = cudaGetDevice(&dev) == cudaSuccess;
@@ -683,29 +697,35 @@ void scratch_give(void* p) {
         std::lock_guard<std::mutex> lock(g_mem_mutex);
         auto it = g_mem_blocks.find(p);
         const size_t bytes = it == g_mem_blocks.end() ? 0 : it->second;
-        if (have && bytes && g_contexts && bytes <= kKeptBytes &&
+        if (have && bytes && g_contexts && (owner || bytes <= kKeptBytes) &&
             !(g_mem_limit && g_mem_used + g_kept_bytes > g_mem_limit)) {
+            if (owner) drop_owned(owner);
             // the newest stays; older ones make room
-            while (!g_kept.empty() && g_kept_bytes + bytes > kKeptBytes) {
-                cudaFree(g_kept.front().p);
-                g_kept_bytes -= g_kept.front().bytes;
-                g_kept.erase(g_kept.begin());
+            for (size_t i = 0; !owner && g_kept_shared + bytes > kKeptBytes;) {
+                if (g_kept[i].owner) ++i;
+                else cudaFree(take_kept(i).p);
             }
             g_mem_blocks.erase(it);
             g_mem_used -= bytes;
-            g_kept.push_back(Kept{p, bytes, dev});
+            g_kept.push_back(Kept{p, bytes, dev, owner});
             g_kept_bytes += bytes;
+            if (!owner) g_kept_shared += bytes;
             return;
         }
     }
     dfree(p);
 }
 
+void scratch_drop(const void* owner) {
+    std::lock_guard<std::mutex> lock(g_mem_mutex);
+    drop_owned(owner);
+}
+
 cudaError_t dmalloc(void** p, size_t bytes) {
     *p = nullptr;
     std::lock_guard<std::mutex> lock(g_mem_mutex);
-    if (g_mem_limit && g_mem_used + g_kept_bytes + bytes > g_mem_limit) drop_kept();
     if (g_mem_limit && g_mem_used + bytes > g_mem_limit) return cudaErrorMemoryAllocation;
+    if (g_mem_limit && g_mem_used + g_kept_bytes + bytes > g_mem_limit) drop_kept();
     cudaError_t e = cudaMalloc(p, bytes);
     if (e == cudaErrorMemoryAllocation && !g_kept.empty()) {
         cudaGetLastError();
@@ -992,7 +1012,8 @@ int wf_destroy(wf_ctx* c) {
     c->tnodes.release(); c->tpairs.release(); c->tinst.release(); c->sinst.release(); c->blas.release(); c->stri.release();
     c->lights.release(); c->aabbs.release(); c->tlas_scratch.release();
     c->tri_albedo.release(); c->inst_tri_offset.release(); c->dimage.release();
-    c->g_albedo.release(); c->g_em_rep.release(); c->L_comp.release(); c->tape.release();
+    c->g_albedo.release(); c->g_em_rep.release(); c->L_comp.release();
+    scratch_drop(c);
     c->image.release(); c->image_ldr.release(); c->trace_io.release(); c->sort_scratch.release();
     dev_free(c->status); dev_free(c->counters); dev_free(c->totals); dev_free(c->trace_fetch);
     for (EventPair& p : c->events) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
@@ -1430,6 +1451,18 @@ std::vector<Wave> plan_waves(uint32_t spp, uint32_t npix, uint32_t wave) {
 // textured frame 2.33 -> 2.40 ms, 720p frame 1.19 -> 1.23 ms).
 constexpr uint32_t kWholePaths = 65536;
 
+// wf_adjoint's recorded hits: kept for the context's next call once the stream
+// is done with them, else (an error on the way) freed, which waits.
+struct Tape {
+    wf_ctx* c;
+    void* p = nullptr;
+    bool done = false;
+    ~Tape() {
+        if (done) scratch_give(p, c);
+        else dfree(p);
+    }
+};
+
 struct Pass {
     WaveParams W;
     SceneRefs S;
@@ -1715,12 +1748,19 @@ int wf_adjoint(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
     };
     auto tape_bytes = [&](uint32_t paths) { return depths * entry * paths; };
     uint32_t tape_wave = tape_paths(4ull << 30);
-    if ((rc = c->tape.reserve(tape_bytes(tape_wave))) == WF_ERR_OOM) {
+    Tape tape{c};
+    cudaError_t te = scratch_take(&tape.p, tape_bytes(tape_wave), c);
+    if (te != cudaSuccess) {
+        cudaGetLastError();
         tape_wave = tape_paths(32ull * c->capacity);
-        rc = c->tape.reserve(tape_bytes(tape_wave));
+        te = scratch_take(&tape.p, tape_bytes(tape_wave), c);
     }
-    if (rc) return rc;
+    if (te != cudaSuccess) {
+        cudaGetLastError();
+        return fail(WF_ERR_OOM, std::string("wf_adjoint: cudaMalloc: ") + cudaGetErrorString(te));
+    }
     wave = tape_wave;
+    uint8_t* const tp = static_cast<uint8_t*>(tape.p);
     std::vector<float4> dimg(npix);
     for (uint32_t p = 0; p < npix; ++p)
         dimg[p] = make_float4(dloss_dimage[3ull * p], dloss_dimage[3ull * p + 1], dloss_dimage[3ull * p + 2], 0.0f);
@@ -1747,9 +1787,9 @@ int wf_adjoint(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
     for (const Wave& wv : plan_waves(o->spp, npix, wave)) {
         // forward pass: each path's radiance and what its rays found
         const uint64_t entries = depths * wv.k * wv.np;
-        P.B.tape_tuvp = reinterpret_cast<float4*>(c->tape.p);
-        P.B.tape_inst = reinterpret_cast<uint32_t*>(c->tape.p + 16 * entries);
-        P.B.tape_clear = c->tape.p + 20 * entries;
+        P.B.tape_tuvp = reinterpret_cast<float4*>(tp);
+        P.B.tape_inst = reinterpret_cast<uint32_t*>(tp + 16 * entries);
+        P.B.tape_clear = tp + 20 * entries;
         if (o->nee) WF_CUDA(cudaMemsetAsync(P.B.tape_clear, 0, entries, c->stream));
         if ((rc = run_wave(c, P, wv, 0, false))) return rc;
         // replay: the same paths from the same seeds and hits, accumulating gradients
@@ -1769,6 +1809,7 @@ int wf_adjoint(wf_ctx* c, const render_settings_t* s, const wf_render_options* o
     }
     if ((rc = end_call(c))) return rc;
     WF_CUDA(cudaStreamSynchronize(c->stream));
+    tape.done = true;
     for (uint64_t t = 0; t < ntri; ++t) {
         d_albedo[3 * t] = ga[t].x;
         d_albedo[3 * t + 1] = ga[t].y;

@@ -56,8 +56,11 @@ cudaError_t dmalloc(void** p, size_t bytes);
 void dfree(void* p);
 // Scratch of a call that has finished with it when it returns (its stream
 // synchronized): a kept block of the current device that fits, else a new one.
-cudaError_t scratch_take(void** p, size_t bytes);
-void scratch_give(void* p);
+// owner: of a context's own block (at most one each), which no other call takes;
+// scratch_drop frees it.
+cudaError_t scratch_take(void** p, size_t bytes, const void* owner = nullptr);
+void scratch_give(void* p, const void* owner = nullptr);
+void scratch_drop(const void* owner);
 int sm_count();
 
 }  // namespace wf
