@@ -1,6 +1,7 @@
 """GPU: the blocks that the library keeps between calls are idle: an adjoint's
 recorded hits do not count as used, make room for other contexts at the memory
-limit and go with their context; all go with the last context."""
+limit and go with their context; at the limit a small build does not take a
+large build's block; all go with the last context."""
 import ctypes
 import os
 import subprocess
@@ -69,6 +70,32 @@ def test_adjoint_hits_are_idle_after_the_call():
         free = torch.cuda.mem_get_info()[0]
         a.close()
         assert torch.cuda.mem_get_info()[0] - free > tape   # with their context, while another lives
+
+
+def test_small_build_leaves_a_large_block_alone_at_the_limit():
+    opts = dict(interval_count=16, max_leaf_prims=4)
+    large, small = scenes.triangle_soup(60_000, seed=1, mu=-3.0), scenes.triangle_soup(2_000, seed=2, mu=-3.0)
+    with Renderer(8, 8) as r:
+        r.bvh_build(small, **opts)
+        base = used()
+        try:
+            # the least room that the large build takes, to 16 KiB
+            lo, hi = 0, 64 << 20
+            while hi - lo > 1 << 14:
+                mid = (lo + hi) // 2
+                limit(1)
+                limit(base + mid)
+                try:
+                    r.bvh_build(large, **opts)
+                    hi = mid
+                except wf.WFError as e:
+                    assert e.status == -2
+                    lo = mid
+            limit(base + hi)
+            r.bvh_build(large, **opts)   # its scratch stays, idle, and fills the limit
+            r.create_mesh_from_triangles(small, **opts)
+        finally:
+            limit(0)
 
 
 LAST = """

@@ -669,9 +669,11 @@ cudaError_t scratch_take(void** p, size_t bytes, const void* owner) {
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) {
         std::lock_guard<std::mutex> lock(g_mem_mutex);
+        // a block counts whole while it is in use: under a limit none of more
+        // than twice the size, which would take other allocations' room
         auto fits = [&](const Kept& k) {
             return k.device == dev && k.owner == owner && k.bytes >= bytes &&
-                   !(g_mem_limit && g_mem_used + k.bytes > g_mem_limit);
+                   !(g_mem_limit && (k.bytes / 2 > bytes || g_mem_used + k.bytes > g_mem_limit));
         };
         size_t best = g_kept.size();
         for (size_t i = 0; i < g_kept.size(); ++i)
