@@ -8,6 +8,7 @@
 // warp reductions take the smallest value and, on equal values, the smallest
 // list position — exactly the element the reference's sequential "area <
 // smallest" loop keeps).
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -359,25 +360,33 @@ __global__ void __launch_bounds__(kScanThreads) k_tlas_build(const float* __rest
     tlas_walk<E>(aabbs, n, nodes, in_smem ? smem : gscratch, metric);
 }
 
-// The walk's launch.  scratch: 7 n words (8 n up to 4,096 instances), used when
+// Lets a kernel that takes at most `most` bytes of dynamic shared memory have
+// `bytes` of it.  48 KiB need no leave, less the kernel's own variables (2 KiB
+// at most here).  Asked for the most, not for the call's own: another thread's
+// smaller build may ask between this and the launch.
+template <class K>
+cudaError_t allow_smem(K kernel, size_t bytes, size_t most) {
+    if (bytes <= 46u * 1024u) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
+// The walk's launch, of a kernel that takes up to `most` instances.  scratch: 7 n words (8 n up to 4,096 instances), used when
 // the list does not fit shared memory (or when smem_ok is false).
 template <class K>
-cudaError_t launch_walk_kernel(K kernel, unsigned T, uint32_t words, const float* aabbs, uint32_t n, float4* nodes,
-                               uint32_t* scratch, uint32_t metric, bool smem_ok, cudaStream_t stream) {
+cudaError_t launch_walk_kernel(K kernel, unsigned T, uint32_t words, const float* aabbs, uint32_t n, uint32_t most,
+                               float4* nodes, uint32_t* scratch, uint32_t metric, bool smem_ok, cudaStream_t stream) {
     const bool in_smem = smem_ok && n <= kSmemInstances;
     const size_t smem = in_smem ? (size_t)n * words * 4u : 0u;
-    if (smem > 48u * 1024u) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(kernel, smem, (size_t)std::min(most, kSmemInstances) * words * 4u);
+    if (e != cudaSuccess) return e;
     kernel<<<1, T, smem, stream>>>(aabbs, n, nodes, scratch, metric, in_smem ? 1 : 0);
     return cudaGetLastError();
 }
 template <uint32_t metric>
 cudaError_t launch_walk(const float* aabbs, uint32_t n, float4* nodes, uint32_t* scratch, bool smem_ok,
                         cudaStream_t st) {
-    auto walk = [&](auto kernel, unsigned threads) {
-        return launch_walk_kernel(kernel, threads, 8u, aabbs, n, nodes, scratch, metric, smem_ok, st);
+    auto walk = [&](auto kernel, unsigned threads, uint32_t most = 1536u) {
+        return launch_walk_kernel(kernel, threads, 8u, aabbs, n, most, nodes, scratch, metric, smem_ok, st);
     };
     // threads by size: us at 64 / 1,025 / 2,048 instances with 32 threads 84 / - / -,
     // 128: 94 / 1,632 / 4,651, 192: 95 / 1,755 / 4,873, 256: 110 / 1,758 / 4,440
@@ -392,9 +401,10 @@ cudaError_t launch_walk(const float* aabbs, uint32_t n, float4* nodes, uint32_t*
         case 109: case 110: return walk(k_tlas_walk<10, 128, metric>, 128);
         case 111: case 112: return walk(k_tlas_walk<12, 128, metric>, 128);
     }
-    if (n <= 2048) return walk(k_tlas_walk<8, 256, metric>, 256);
-    if (n <= 4096) return walk(k_tlas_walk<16, 256, metric>, 256);
-    return launch_walk_kernel(k_tlas_build<4>, kScanThreads, 7u, aabbs, n, nodes, scratch, metric, smem_ok, st);
+    if (n <= 2048) return walk(k_tlas_walk<8, 256, metric>, 256, 2048);
+    if (n <= 4096) return walk(k_tlas_walk<16, 256, metric>, 256, 4096);
+    return launch_walk_kernel(k_tlas_build<4>, kScanThreads, 7u, aabbs, n, kSmemInstances, nodes, scratch, metric,
+                              smem_ok, st);
 }
 
 }  // namespace
@@ -1441,10 +1451,8 @@ cudaError_t launch_tlas_build(const float* aabbs, uint32_t n, float4* nodes, uin
         const uint32_t P = pow2_at_least(n);
         const bool smem = n <= kPlocSmemMax;
         const size_t bytes = smem ? ploc_bytes(n, P) : 0;
-        if (bytes > 48u * 1024u) {
-            cudaError_t e = cudaFuncSetAttribute(k_tlas_ploc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e != cudaSuccess) return e;
-        }
+        const cudaError_t e = allow_smem(k_tlas_ploc, bytes, ploc_bytes(kPlocSmemMax, kPlocSmemMax));
+        if (e != cudaSuccess) return e;
         k_tlas_ploc<<<1, kPlocThreads, bytes, stream>>>(aabbs, n, nodes, scratch, P, smem);
         return cudaGetLastError();
     }
@@ -1454,10 +1462,8 @@ cudaError_t launch_tlas_build(const float* aabbs, uint32_t n, float4* nodes, uin
         const uint32_t P = pow2_at_least(n);
         const bool smem = n <= kSweepSmemMax;
         const size_t bytes = smem ? 4 * sweep_words(n, P) : 0;
-        if (bytes > 48u * 1024u) {
-            cudaError_t e = cudaFuncSetAttribute(k_tlas_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e != cudaSuccess) return e;
-        }
+        const cudaError_t e = allow_smem(k_tlas_sweep, bytes, 4 * sweep_words(kSweepSmemMax, kSweepSmemMax));
+        if (e != cudaSuccess) return e;
         k_tlas_sweep<<<1, kPlocThreads, bytes, stream>>>(aabbs, n, nodes, scratch, P, smem);
         return cudaGetLastError();
     }
