@@ -175,9 +175,9 @@ def measured_peaks():
 
 def ncu_traffic(rays_per_launch):
     """DRAM bytes per extension launch from the committed ncu summary
-    (profiles/extend_instanced_1080p.json: read + written bytes per ray over
-    the nine extension launches of a reduced frame, and the git commit it was
-    captured at), scaled to this frame's rays per launch."""
+    (profiles/extend_instanced_1080p.json: read + written bytes per traced ray
+    over the nine extension launches of a reduced frame, and the git commit it
+    was captured at), scaled to this frame's traced rays per launch."""
     p = os.path.join(ROOT, "profiles", "extend_instanced_1080p.json")
     if not os.path.exists(p):
         return None, None
@@ -591,9 +591,21 @@ def run_ours(args, rank, world, local):
     r.render(max_bounces=DEPTH, spp=SPP, frame_seed=1, nee=1, rr_start_depth=RR, accumulate=False,
              count_traffic=True)
     c = r.stats()
-    alg_bytes = (c["rays_extend"] * (B_RAY + B_HIT) + c["tlas_node_loads"] * B_TNODE + c["instance_loads"] * B_INST
-                 + c["blas_node_loads"] * B_BNODE + c["triangle_tests"] * B_TRI)
-    alg_bytes -= c["paths"] * B_RAY   # camera rays are made in the depth-0 launch, not read
+    # the timed frames trace one camera ray per pixel (one wave holds a frame's
+    # samples), the counted pass each sample's own, all alike
+    def traced(d):
+        """Extension rays traced at depth d."""
+        n = int(c["extend_rays_depth"][d])
+        return n // SPP if d == 0 else n
+
+    def extend_bytes(d):
+        """Algorithmic bytes of the extension rays of depth d (the counted
+        pass); camera rays are made in their launch, not read."""
+        n, f = int(c["extend_rays_depth"][d]), c["extend_fetch_depth"][d]
+        b = (n * (B_HIT + (0 if d == 0 else B_RAY)) + f[0] * B_TNODE + f[1] * B_INST + f[2] * B_BNODE
+             + f[3] * B_TRI)
+        return b / SPP if d == 0 else b
+
     def shadow_bytes(d):
         """Algorithmic bytes of the shadow rays of depth d (the counted pass)."""
         f = c["shadow_fetch_depth"][d]
@@ -602,19 +614,17 @@ def run_ours(args, rank, world, local):
 
     # from this depth on, an extension launch also traces the previous depth's shadow rays
     fuse_from = 1 if args.fused_connect else args.fused_from_depth
-    if fuse_from:
-        alg_bytes += sum(shadow_bytes(d - 1) for d in range(max(1, fuse_from), DEPTH + 1))
     # the launches measured are the staged extension launches: with a tail, the
-    # rays of its depths (under 1 % of them on this frame) leave the count
-    tail_d = int(last["tail_depth"])
-    if tail_d:
-        q = [int(x) for x in c["extend_rays_depth"][:DEPTH + 1]]
-        alg_bytes = alg_bytes * sum(q[:tail_d]) / max(1, sum(q))
+    # rays of its depths (under 1 % of them on this frame) are not among them
+    staged = range(int(last["tail_depth"]) or DEPTH + 1)
+    alg_bytes = sum(extend_bytes(d) for d in staged)
+    if fuse_from:
+        alg_bytes += sum(shadow_bytes(d - 1) for d in staged if d >= max(1, fuse_from))
     bytes_per_launch = alg_bytes / max(1, ext_launches / args.steps)
     ms_per_launch = ext_ms / max(1, ext_launches)
     achieved = bytes_per_launch / (ms_per_launch / 1e3) / 1e9
     peak, peak_kind = measured_peaks()
-    traffic, traffic_src = ncu_traffic(c["rays_extend"] / max(1, ext_launches / args.steps))
+    traffic, traffic_src = ncu_traffic(sum(traced(d) for d in staged) / max(1, ext_launches / args.steps))
     # per depth: the extension launches (depth 0 makes its camera rays) and the
     # shadow-ray launches, algorithmic bytes of the counted pass over the
     # timed frames' CUDA-event time of that depth's launch
@@ -627,12 +637,12 @@ def run_ours(args, rank, world, local):
             n_d, f = int(c["extend_rays_depth"][d]), c["extend_fetch_depth"][d]
             ms_d = ext_ms_d[d] / frames
             if n_d and ms_d > 0:
-                b = (n_d * (B_HIT + (0 if d == 0 else B_RAY)) + f[0] * B_TNODE + f[1] * B_INST + f[2] * B_BNODE
-                     + f[3] * B_TRI)
+                b = extend_bytes(d)
                 fused = fuse_live and fuse_from and d >= max(1, fuse_from)
                 if fused:
                     b += shadow_bytes(d - 1)   # the launch also traced the shadow rays of depth d - 1
-                ext_rows.append({"depth": d, "rays": n_d, "alg_bytes": int(b), "ms": round(ms_d, 4),
+                ext_rows.append({"depth": d, "rays": n_d, "rays_traced": traced(d), "alg_bytes": int(b),
+                                 "ms": round(ms_d, 4),
                                  **({"with_shadow_rays_of_depth": d - 1} if fused else {}),
                                  "achieved_gbs": round(b / (ms_d / 1e3) / 1e9, 1),
                                  "frac": round(b / (ms_d / 1e3) / 1e9 / peak, 4),
@@ -804,6 +814,7 @@ def run_ours(args, rank, world, local):
                 "rays_per_step": rays // args.steps,
                 # without the camera rays that share another path's (one wave holds a frame's samples)
                 "rays_traced_per_step": rays // args.steps - (c["paths"] - W * H),
+                "traced_mrays_per_s": round(value * (1.0 - (c["paths"] - W * H) * args.steps / max(1, rays)), 3),
                 "gpu_launches": launches,
                 "stages_ms": {k: round(last[f"ms_{k}"], 3) for k in ("generate", "extend", "shade", "connect", "post",
                                                                         "tail")},
@@ -832,8 +843,7 @@ def run_ours(args, rank, world, local):
                              "achieved": round(achieved, 1),
                              "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                              "frac": round(achieved / peak, 4), "traffic": traffic, "traffic_source": traffic_src,
-                             # depth 0 carries 74 % of the counted rays: the 16 camera rays of a pixel are one
-                             # traced ray, whose fetches count 16 times; the secondary depths are the real traversal
+                             # bytes of the rays that are traced: a pixel's camera rays are one
                              "per_depth": per_depth, "frac_secondary": secondary["frac"] if secondary else None,
                              "secondary": secondary, "connect": connect, "solo": solo,
                              "alg_bytes_per_launch": int(bytes_per_launch),
