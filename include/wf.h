@@ -161,8 +161,10 @@ typedef struct wf_render_options {
      * depth.  0 = never (the default: with next-event estimation a path's
      * shadow and extension rays then wait for each other, where the staged
      * launches overlap them; textured and instanced frames took 3-5 % longer).
-     * Waves of at most 65,536 paths that cast no shadow rays run whole in that
-     * launch whatever this is.  Images are identical either way. */
+     * With 0, waves of at most 65,536 paths that cast no shadow rays run whole
+     * in that launch, from their camera rays on: over the binary BLAS layout,
+     * without a debug view, profile or count_traffic (which time and count the
+     * staged launches).  Images are identical either way. */
     uint32_t tail_paths;
     /* WF_SCHEDULE_SEPARATE only: from this depth (>= 1) on, the extension
      * launch of depth d also traces the shadow rays of depth d - 1, as the
@@ -211,7 +213,8 @@ typedef struct wf_stats {
     /* the tail (wf_render_options.tail_paths): GPU time of its launches
      * (profile = 1; not in ms_extend) and the depth at which the last wave
      * handed its remaining bounces to it (0 = the wave ran every depth in
-     * stages; a tail launch counts in launches, not in launches_extend) */
+     * stages, or whole in one launch; a launch of either kind counts in
+     * launches, not in launches_extend) */
     double   ms_tail;
     uint64_t tail_depth;
     /* profile = 1: GPU time of the extension (incl. the depth-0 camera rays)
@@ -355,7 +358,8 @@ int wf_scene_set_emission(wf_ctx* ctx, uint32_t instance, float strength);
  * replay takes the forward pass's decisions): the gradient of the expected
  * image stays unbiased.  Metal and dielectric base colours are not
  * differentiated, nor an albedo of exactly 0 (its path carries nothing
- * further).  Requires wf_scene_set_albedo; the shadow rays are traced in
+ * further).  The statistics count the rays of the forward pass, the only ones
+ * traced.  Requires wf_scene_set_albedo; the shadow rays are traced in
  * their own launches whatever trace_schedule says. */
 int wf_adjoint(wf_ctx* ctx, const render_settings_t* settings, const wf_render_options* opts, uint32_t frame_seed,
                const float* dloss_dimage, float* d_albedo, float* d_emission);

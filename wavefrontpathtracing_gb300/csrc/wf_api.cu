@@ -1443,10 +1443,13 @@ std::vector<Wave> plan_waves(uint32_t spp, uint32_t npix, uint32_t wave) {
 // Waves of at most this many paths without shadow rays run whole in one
 // k_finish launch instead of an extend and a shade launch per depth.  us per
 // frame, staged / whole, frames of three contexts in flight (alone), box scene
-// depth 4: 4,096 paths 181 / 107 (374 / 228), 32,761: 252 / 185 (477 / 347),
-// 65,536: 299 / 235 (550 / 416), 131,044: 365 / 380 (652 / 617), 262,144:
-// 509 / 711; five spheres of every material, depth 8: 65,536: 554 / 495,
-// 131,072: 689 / 810.  (k_finish keeps 77,824 paths in flight: 4 blocks of 128
+// depth 4: 4,096 paths 165 / 92 (349 / 200), 32,761: 219 / 143 (428 / 273),
+// 65,536: 253 / 175 (470 / 323), 108,900: 287 / 237 (514 / 431), 131,044: 302 /
+// 278 (543 / 467), 160,000: 322 / 331 (581 / 498), 262,144: 399 / 520 (659 /
+// 682); five spheres of every material, depth 8: 65,536: 455 / 355 (750 / 488),
+// 131,072: 553 / 573 (871 / 768), 262,144: 785 / 1,130; 300 instances of small
+// spheres: 65,536: 186 / 128, 262,144: 265 / 197.  So the line lies below every
+// scene's crossing.  (k_finish keeps 77,824 paths in flight: 4 blocks of 128
 // on each of 152 SMs.)  With shadow rays a path's own chain is twice as long
 // and the staged launches overlap their two kinds: from the first queue of at
 // most 65,536 paths on, finishing a wave measured 3-5 % slower there (613x377

@@ -357,8 +357,9 @@ __device__ __forceinline__ void bins_reset(uint32_t* sb, uint32_t words, uint32_
 // with the level's node count read back by the host, took about 100 us per
 // level however few triangles it had; us per wf_bvh_build, so / in one launch,
 // with the renumbering below: 80 triangles 296 / 190, 1,280: 672 / 356, 20,480:
-// 1,634 / 851, 100,820: 2,684 / 1,560, 499,280: 7,423 / 6,180 (0.98 ms of it
-// k_large, 0.97 k_small, most of the rest the host's).
+// 1,634 / 851, 100,820: 2,684 / 1,560, 499,280: 7,423 / 6,180 (1.00 ms of it
+// k_large, 0.98 k_small, most of the rest the host's; 4,450 to 6,000 by the state
+// of the caller's output pages since the positions are picked out on the GPU).
 //
 // A slot is a node of the level, a chunk kChunk consecutive positions of one
 // slot; a block takes chunks in turn.  Slots and chunks of the next level are

@@ -155,9 +155,9 @@ __global__ void __launch_bounds__(kShadeBlock, MODE == kViews ? 2 : WF_SHADE_MIN
 //
 // Bound by the gathers of shade_one and the albedo atomics.  A 512x512 x 64
 // sample adjoint of depth 6 took 70.6 ms with a replay that traced every ray
-// again through the staged launches, 39.2 ms so (blocks of 256, 2 / 3 resident:
-// 39.3 / 39.4; 128, 7 resident: 39.3).
-// (All with single-float albedo atomics and an earlier traversal loop; 29.2 ms now.)
+// again through the staged launches, 39.2 ms so on the traversal loop of that
+// time and 28.9 ms now.  3 / 4 / 5 / 6 / 7 resident blocks: 29.5 / 29.5 / 28.9 /
+// 28.8 / 28.6 ms, with next-event estimation 50.7 / 50.7 / 50.7 / 50.9 / 50.9.
 constexpr int kReplayBlock = 128, kReplayMinBlocks = 5;
 __global__ void __launch_bounds__(kReplayBlock, kReplayMinBlocks)
     k_replay(ShadeRefs SH, RenderBuffers B, WaveParams W, AdjointRefs A) {

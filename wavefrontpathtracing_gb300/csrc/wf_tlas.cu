@@ -1479,8 +1479,8 @@ cudaError_t launch_tlas_build(const float* aabbs, uint32_t n, float4* nodes, uin
 // or an engine that hands out all of its device memory from a budget fixed up
 // front (its own pool, a hard memory cap).  They pass their own
 // device buffers for the instance boxes and the output nodes; the build's
-// working list (7 words per instance) lives in one fixed-size static device
-// array that every call on a device shares.
+// working list (8 words per instance up to 4,096 instances, else 7) lives in
+// one fixed-size static device array that every call on a device shares.
 
 namespace {
 

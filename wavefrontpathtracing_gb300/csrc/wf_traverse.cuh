@@ -39,7 +39,10 @@
 // frame 222 -> 172 us; then nodes and instance rows in 32-byte loads, half the
 // requests: 9.53 ms, 1.02, 298 us, 4.46 ms, and with new rays at 12 idle lanes
 // again 9.29, 1.02, 290, 4.44 (quantized and exact 4-wide: 6.02 ->
-// 6.01, 7.04 -> 6.07).
+// 6.01, 7.04 -> 6.07).  Each pair on one GPU; the 1M any-hit rays take 232 to
+// 290 us from GPU to GPU, so their small steps show little by themselves.  One
+// ray alone over a 4-wide layout takes 37 us where a step per iteration took 34
+// (eight rays: 69 and 82).
 #pragma once
 #include <type_traits>
 #include "wf_device.cuh"
