@@ -1225,8 +1225,10 @@ int gpu_bvh_build(const triangle_t* tris, uint32_t n, const wf_bvh_options& o, c
         void* args[] = {&C, &G};
         BVH_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_large), dim3(grid), dim3(kChunkThreads), args, 0, st));
     }
+    // under the 48 KiB that need no leave: asking for a call's own size would
+    // set another thread's maximum
+    static_assert(small_smem_bytes(kMaxBins) <= 46u * 1024u, "");
     const size_t smem = small_smem_bytes(B);
-    BVH_CUDA(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_small<<<blocks_for(n, 48, 1u << 16), 32 * kSmallWarps, smem, st>>>(C, (uint32_t)tcap);
     BVH_CUDA(cudaMemsetAsync(arrived, 0, 4ull * tcap, st));
     k_count<<<blocks_for(tcap, 256), 256, 0, st>>>(C, arrived, ic, up);
