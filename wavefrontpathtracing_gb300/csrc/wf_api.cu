@@ -989,10 +989,15 @@ int wf_create(const wf_init_params* p, wf_ctx** out) {
     if (rc == WF_OK) rc = dev_alloc(&c->trace_fetch, 1);
     if (rc == WF_OK) rc = dev_alloc(&c->totals, 2 + 2 * kMaxDepth);
     if (rc == WF_OK) {
-        cudaMemset(c->status, 0, 4);
-        cudaMemset(c->counters, 0, 2 * kMaxDepth * sizeof(Counters));
-        cudaMemset(c->totals, 0, (2 + 2 * kMaxDepth) * sizeof(unsigned long long));
-        if (cudaDeviceSynchronize() != cudaSuccess) rc = fail(WF_ERR_CUDA, "wf_create: device initialization failed");
+        // on the context's own stream: another thread may be capturing a batch's graph,
+        // which a wait for the whole device would refuse and break
+        if (cudaMemsetAsync(c->status, 0, 4, c->stream) != cudaSuccess ||
+            cudaMemsetAsync(c->counters, 0, 2 * kMaxDepth * sizeof(Counters), c->stream) != cudaSuccess ||
+            cudaMemsetAsync(c->totals, 0, (2 + 2 * kMaxDepth) * sizeof(unsigned long long), c->stream) != cudaSuccess ||
+            cudaStreamSynchronize(c->stream) != cudaSuccess) {
+            cudaGetLastError();
+            rc = fail(WF_ERR_CUDA, "wf_create: device initialization failed");
+        }
     }
     if (rc != WF_OK) {
         wf_destroy(c);
