@@ -145,25 +145,29 @@ __global__ void __launch_bounds__(kShadeBlock, MODE == kViews ? 2 : WF_SHADE_MIN
 // again from the hit that the forward pass recorded, so no ray is traced and no
 // queue written; the path's state and its radiance so far (with its rounding
 // errors) stay in registers, summed in the forward pass's order.  The gradients
-// go out as shade_one's atomics, the emitters' into 32 replicas (a shadow ray's
-// contribution by path, the emitter a path ends at once per warp).  One number
+// go out as shade_one's atomics, the emitters' into 32 replicas: a path sums its
+// terms of one emitter, a shadow ray's and the emission it ends at, and a warp
+// its paths'.  One number
 // per emitter sums millions of terms whose signs cancel where the image
-// gradient's do, so warps and replicas add in double: over 12 image gradients
-// of the adjoint below, 1e-8 to 1.1e-6 from the FP64 sum over the image, against
-// 2e-7 to 2.4e-5 with float replicas and up to 5e-5 with one float per emitter
-// (28.86 ms against 28.80).
+// gradient's do, so paths, warps and replicas add in double: over 12 image
+// gradients of the adjoint below, 1e-8 to 1.1e-6 from the FP64 sum over the
+// image, against 2e-7 to 2.4e-5 with float replicas and up to 5e-5 with one
+// float per emitter.  (An atomic per shadow ray instead took 50.7 ms with
+// next-event estimation, 43.1 so; without, where the kernel leaves that code out,
+// 28.85 and 28.10.)
 //
 // Bound by the gathers of shade_one and the albedo atomics.  A 512x512 x 64
 // sample adjoint of depth 6 took 70.6 ms with a replay that traced every ray
 // again through the staged launches, 39.2 ms so on the traversal loop of that
-// time and 28.9 ms now.  3 / 4 / 5 / 6 / 7 resident blocks: 29.5 / 29.5 / 28.9 /
-// 28.8 / 28.6 ms, with next-event estimation 50.7 / 50.7 / 50.7 / 50.9 / 50.9.
+// time and 28.0 ms now.  4 / 5 / 6 / 7 resident blocks: 28.04 / 28.03 / 28.08 /
+// 27.87 ms, with next-event estimation 43.98 / 43.04 / 42.94 / 42.83.
 constexpr int kReplayBlock = 128, kReplayMinBlocks = 5;
+template <bool NEE>
 __global__ void __launch_bounds__(kReplayBlock, kReplayMinBlocks)
     k_replay(ShadeRefs SH, RenderBuffers B, WaveParams W, AdjointRefs A) {
     const uint32_t path = blockIdx.x * kReplayBlock + threadIdx.x;
     ShadeCtl K;
-    K.frame_seed = W.frame_seed; K.max_bounces = W.max_bounces; K.nee = W.nee; K.rr_start = W.rr_start;
+    K.frame_seed = W.frame_seed; K.max_bounces = W.max_bounces; K.nee = NEE ? 1u : 0u; K.rr_start = W.rr_start;
     K.cosine = W.cosine; K.env_strength = W.env_strength; K.env0 = W.env[0]; K.env1 = W.env[1]; K.env2 = W.env[2];
     K.lights = SH.lights; K.light_count = SH.light_count; K.light_total = SH.light_total;
     K.env_tex = W.env_tex; K.view_mode = 0u; K.far_plane = W.far_plane;
@@ -186,6 +190,14 @@ __global__ void __launch_bounds__(kReplayBlock, kReplayMinBlocks)
             in.Lb.y = two_sum(in.Lb.y, c.y, e); in.Lb_lo.y = in.Lb_lo.y + e;
             in.Lb.z = two_sum(in.Lb.z, c.z, e); in.Lb_lo.z = in.Lb_lo.z + e;
         };
+        auto emitted = [&](uint32_t key, float v) {
+            if (key != em_key) {
+                if (em_key != kInvalid) atomicAdd(&A.g_em_rep[(size_t)(path & 31u) * A.instances + em_key], em_val);
+                em_key = key;
+                em_val = 0.0;
+            }
+            em_val += v;
+        };
         for (uint32_t depth = 0; depth <= W.max_bounces; ++depth) {
             const size_t at = (size_t)depth * W.npaths + path;
             in.tuvp = B.tape_tuvp[at];
@@ -194,8 +206,8 @@ __global__ void __launch_bounds__(kReplayBlock, kReplayMinBlocks)
             ShadeOut o;
             shade_one(SH, K, in, A, path, in.pixel, o);
             if (o.has_add) gather(o.add);
-            if (o.em_key != kInvalid) { em_key = o.em_key; em_val = o.em_val; }   // the path ends at an emitter
-            if (o.shadow && B.tape_clear[at]) {
+            if (o.em_key != kInvalid) emitted(o.em_key, o.em_val);   // the path ends at an emitter
+            if (NEE && o.shadow && B.tape_clear[at]) {
                 gather(o.contrib);
                 // linear in the emitter's strength
                 if (in_bounds(o.light_inst, A.instances, B.status)) {
@@ -204,8 +216,7 @@ __global__ void __launch_bounds__(kReplayBlock, kReplayMinBlocks)
                         const float4 g = A.dimage[in.pixel];
                         const float v = (g.x * A.inv_spp) * o.contrib.x + (g.y * A.inv_spp) * o.contrib.y +
                                         (g.z * A.inv_spp) * o.contrib.z;
-                        atomicAdd(&A.g_em_rep[(size_t)(path & 31u) * A.instances + o.light_inst],
-                                  (double)(v / strength));
+                        emitted(o.light_inst, v / strength);
                     }
                 }
             }
@@ -292,7 +303,8 @@ cudaError_t launch_shade(const ShadeRefs& SH, const RenderBuffers& B, const Wave
 
 cudaError_t launch_replay(const ShadeRefs& SH, const RenderBuffers& B, const WaveParams& W, const AdjointRefs& A,
                           cudaStream_t stream) {
-    k_replay<<<(W.npaths + kReplayBlock - 1) / kReplayBlock, kReplayBlock, 0, stream>>>(SH, B, W, A);
+    const auto replay = W.nee ? k_replay<true> : k_replay<false>;
+    replay<<<(W.npaths + kReplayBlock - 1) / kReplayBlock, kReplayBlock, 0, stream>>>(SH, B, W, A);
     return cudaGetLastError();
 }
 
